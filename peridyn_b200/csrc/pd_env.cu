@@ -84,6 +84,10 @@ pd::Geo pd_env::geo() const {
     g.nbr = nbr.p;
     g.fam = fam.p;
     g.deformed = deformed.p;
+    g.max_slots = max_slots;
+    g.has_ep = 0;
+    for (const auto &b : hb)
+        if (b.kind == PD_MAT_ELASTO_PLASTIC) g.has_ep = 1;
     g.td2 = td2.p;
     g.edp_in = edp[ecur].p;
     g.edp_out = edp[1 - ecur].p;
@@ -652,6 +656,7 @@ static pd_status build_runtime_layout(pd_env *env, const std::vector<int64_t> &s
     env->cnt_h = cnt;
     env->nnz = (int64_t)kSlice * nwords;
     env->walked = walked_slots(env->cnt_h);
+    env->max_slots = env->cnt_h.empty() ? 0 : *std::max_element(env->cnt_h.begin(), env->cnt_h.end());
     env->nbr_len = nbr_len;
     env->stencil_slices = nst;
     cudaStream_t st = env->st;
@@ -760,6 +765,7 @@ static pd_status build_runtime_layout_device(pd_env *env, const std::vector<int6
     env->cnt_h = cnt_b;
     env->nnz = (int64_t)kSlice * nwords;
     env->walked = walked_slots(env->cnt_h);
+    env->max_slots = env->cnt_h.empty() ? 0 : *std::max_element(env->cnt_h.begin(), env->cnt_h.end());
     env->nbr_len = nbr_len;
     env->stencil_slices = nst;
     return PD_OK;

@@ -9,9 +9,11 @@
 //   get_ij         x[:, j] - x[:, i]                   const_macros.jl:153-155
 //   stretch        (|Y| - |X|) / |X|                   general_material.jl:338-341
 //   force          ((0.5*t/|Y|) * Y_d * V_j) / rho_i   general_material.jl:351-362
+#include <atomic>
 #include <climits>
 #include <cstdio>
 
+#include "pd_ieee.h"
 #include "pd_internal.h"
 
 namespace pd {
@@ -27,6 +29,13 @@ inline unsigned grid_for(int64_t n, int threads = kThreads) {
 
 __device__ __forceinline__ double mag3(double a1, double a2, double a3) {
     return sqrt(a1 * a1 + a2 * a2 + a3 * a3);
+}
+
+// One 256-bit load of a particle's record.
+__device__ __forceinline__ double4 ld4(const double4 *p) {
+    double4 r;
+    asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+    return r;
 }
 
 __device__ __forceinline__ int64_t sell_base(const int64_t *slice_ptr, int64_t p) {
@@ -297,33 +306,80 @@ __global__ void k_weighted_volume(Geo g, double2 *__restrict__ mth) {
 // peri.jl:155-172 dilatation!: theta_i = sum over intact bonds, in family
 // order, of (((3/m_i) * w) * |X|) * e * V_j  (horizon correction == 1).
 // ---------------------------------------------------------------------
-__global__ void k_theta_serial(Geo g, const double4 *__restrict__ y,
-                               const uint32_t *__restrict__ win, double2 *__restrict__ mth,
-                               int64_t p0, int64_t p1) {
-    int64_t p = p0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (p >= p1) return;
-    int32_t ti = g.tinfo[p];
-    if (ti < 0) return;
-    const DevBlock &B = g.blocks[ti >> 8];
-    if (B.kind != PD_MAT_ORDINARY_STATE_BASED && B.kind != PD_MAT_ELASTO_PLASTIC) return;
-    double4 xp = g.x4[p], yp = y[p];
-    double c_i = 3.0 / mth[p].x;
-    int32_t n = g.cnt[p];
-    const BondRef br = bond_ref(g.si, g.nbr, win, p);
+// The operators' evaluation of a term the branch-free one does not cover.
+__device__ __noinline__ double theta_term_general(double4 xp, double4 yp, double4 xq, double4 yq, double c_i) {
+    const double xij = mag3(xq.x - xp.x, xq.y - xp.y, xq.z - xp.z);
+    const double yij = mag3(yq.x - yp.x, yq.y - yp.y, yq.z - yp.z);
+    const double e = yij - xij;
+    const double wi = 1.0 / xij;
+    return c_i * wi * xij * e * xq.w;
+}
+
+// One block per slice: the warps evaluate the terms of the slice's slots
+// side by side (tiles of kThetaTile slots in shared memory, a contiguous run
+// of a tile's slots per warp, two slots at a time), then one warp adds them
+// in family order.  Slots without an intact bond hold zero (the sum starts
+// at +0.0 and so is never -0.0).  A thread per particle, one term after
+// another, took 102 us on the 40,000-particle bar, this kernel 29 us.
+constexpr int32_t kThetaTile = 128;
+template <int NW>
+__global__ void __launch_bounds__(32 * NW, NW == 8 ? 3 : 1)
+    k_theta_slice(Geo g, const double4 *__restrict__ y, const uint32_t *__restrict__ win, double2 *__restrict__ mth,
+                  int64_t s0) {
+    __shared__ double term[kThetaTile][32];
+    const int64_t s = s0 + blockIdx.x;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t p = 32 * s + lane;
+    const int32_t ti = g.tinfo[p];
+    const int32_t tb = __reduce_max_sync(0xffffffffu, ti);
+    const int kind = tb >= 0 ? g.blocks[tb >> 8].kind : PD_MAT_SKIP;
+    if (kind != PD_MAT_ORDINARY_STATE_BASED && kind != PD_MAT_ELASTO_PLASTIC) return;
+    const double4 xp = ld4(g.x4 + p), yp = ld4(y + p);
+    const double c_i = ti >= 0 ? 3.0 / mth[p].x : 0.0;
+    const int32_t n = g.cnt[p];
+    const int32_t L = (int32_t)__reduce_max_sync(0xffffffffu, (unsigned)n);
+    const SliceInfo d = g.si[s];
+    const bool st = d.mode == kStencil;
+    const int32_t *nb = g.nbr + d.nbr + (st ? 0 : lane);
+    const uint32_t *wi = win + d.word + lane;
+    auto neighbour = [&](int32_t k) -> int32_t {
+        if (k >= n) return (int32_t)p;
+        return st ? (int32_t)p + __ldg(nb + k) : __ldg(nb + 32 * k);
+    };
+    auto evaluate = [&](const double4 &xq, const double4 &yq, double &t) -> bool {
+        const double X1 = xq.x - xp.x, X2 = xq.y - xp.y, X3 = xq.z - xp.z;
+        const double Y1 = yq.x - yp.x, Y2 = yq.y - yp.y, Y3 = yq.z - yp.z;
+        double xij, yij, rx, ry;
+        bool fast = sqrt_rcp_rn(X1 * X1 + X2 * X2 + X3 * X3, xij, rx);
+        fast = sqrt_rcp_rn(Y1 * Y1 + Y2 * Y2 + Y3 * Y3, yij, ry) && fast;
+        t = c_i * rx * xij * (yij - xij) * xq.w;
+        return fast;
+    };
     double th = 0.0;
-    uint32_t w = 0;
-    for (int32_t k = 0; k < n; ++k) {
-        if ((k & 31) == 0) w = *br.word(k);
-        if (!((w >> (k & 31)) & 1u)) continue;
-        int32_t q = br.q(k);
-        double4 xq = g.x4[q], yq = y[q];
-        double xij = mag3(xq.x - xp.x, xq.y - xp.y, xq.z - xp.z);
-        double yij = mag3(yq.x - yp.x, yq.y - yp.y, yq.z - yp.z);
-        double e = yij - xij;
-        double wi = 1.0 / xij;
-        th = th + c_i * wi * xij * e * xq.w;
+    for (int32_t base = 0; base < L; base += kThetaTile) {
+        const int32_t m = min(kThetaTile, L - base);
+        const int32_t per = (m + NW - 1) / NW, j0 = min(w * per, m), j1 = min(j0 + per, m);
+        if (base) __syncthreads();
+        for (int32_t j = j0; j < j1; j += 2) {
+            const int32_t ka = base + j, kb = base + min(j + 1, j1 - 1);
+            const int32_t qa = neighbour(ka), qb = neighbour(kb);
+            const bool la = ka < n && ((wi[32 * (ka >> 5)] >> (ka & 31)) & 1u);
+            const bool lb = kb < n && ((wi[32 * (kb >> 5)] >> (kb & 31)) & 1u);
+            const double4 xa = ld4(g.x4 + qa), ya = ld4(y + qa), xb = ld4(g.x4 + qb), yb = ld4(y + qb);
+            double ta, tb2;
+            const bool ea = evaluate(xa, ya, ta), eb = evaluate(xb, yb, tb2);
+            if (la && !ea) ta = theta_term_general(xp, yp, xa, ya, c_i);
+            if (lb && !eb) tb2 = theta_term_general(xp, yp, xb, yb, c_i);
+            term[j][lane] = la ? ta : 0.0;
+            if (j + 1 < j1) term[j + 1][lane] = lb ? tb2 : 0.0;
+        }
+        __syncthreads();
+        if (w == 0) {
+#pragma unroll 8
+            for (int32_t j = 0; j < m; ++j) th = th + term[j][lane];
+        }
     }
-    mth[p].y = th;
+    if (w == 0 && ti >= 0) mth[p].y = th;
 }
 
 // One bond term seen from particle p: returns true when the bond is
@@ -577,12 +633,18 @@ __device__ void force_serial_particle(const Geo &g, int64_t p, int32_t ti,
     f[p] = make_double4(fx, fy, fz, 0.0);
 }
 
+// The slots a 32-particle slice walks: the largest slot count of its lanes.
+__device__ __forceinline__ int32_t slice_slots(int32_t n) { return (int32_t)__reduce_max_sync(0xffffffffu, (unsigned)n); }
+
+// One thread per particle, every bond evaluated from both visits: the
+// elasto-plastic blocks (whose two visits differ) and slices with more than
+// cap slots.  The other slices belong to k_force_slice.
 __global__ void __launch_bounds__(kThreads)
     k_force_serial(Geo g, const double4 *__restrict__ y, const double2 *__restrict__ mth,
                    const uint32_t *__restrict__ win, uint32_t *__restrict__ wout,
-                   double4 *__restrict__ f, int accumulate, int64_t p0, int64_t p1) {
+                   double4 *__restrict__ f, int accumulate, int32_t cap, int64_t p0, int64_t p1) {
     int64_t p = p0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (p >= p1) return;
+    if (p >= p1) return;  // whole warps: p0 and p1 are multiples of 32
     int32_t ti = g.tinfo[p];
     int32_t n = g.cnt[p];
     const int64_t wb = g.si[p >> 5].word + (p & 31);
@@ -593,6 +655,7 @@ __global__ void __launch_bounds__(kThreads)
         kind = B.kind;
         active = kind != PD_MAT_SKIP && g.deformed[ti >> 8] != 0;
     }
+    if (!__any_sync(0xffffffffu, kind == PD_MAT_ELASTO_PLASTIC) && slice_slots(n) <= cap) return;
     if (!active) {
         for (int32_t w = 0; w * 32 < n; ++w) wout[wb + 32 * (int64_t)w] = win[wb + 32 * (int64_t)w];
         if (kind == PD_MAT_ELASTO_PLASTIC && g.edp_out)
@@ -607,6 +670,270 @@ __global__ void __launch_bounds__(kThreads)
     else
         force_serial_particle<PD_MAT_ORDINARY_STATE_BASED>(g, p, ti, y, mth, win, wout, f,
                                                             accumulate);
+}
+
+// ---------------------------------------------------------------------
+// The same sums with every bond evaluated once, one block per slice.  The
+// PMB and LPS terms are the same number from either visit, so only the
+// order of the additions is serial: the block's warps evaluate the slice's
+// slots side by side (warp w takes the w-th run of slots) into shared
+// memory, 24 bytes per slot and lane, and then one warp per component adds
+// them in the order A, B, C above.  A slot without a term holds a zero,
+// which changes no partial sum: x + 0 == x unless x is -0.0, and a sum of
+// at least one nonnegative-zero start is never -0.0 (slices whose caller
+// passes -0.0 in f take the particle loop).
+//
+// What bounds it: the two blocks an SM holds (94 KB of terms for 122 slots)
+// alternate between evaluation, a chain of some 600 cycles per pair of
+// slots, and the sums, 244 dependent additions of 17 cycles.  FP64 pipe 33 %,
+// issue 47 % busy (48^3 PMB cube).  Against a thread per particle
+// that evaluates a bond at each of its two visits: force pass of a
+// 990-particle cube 15 against 198 us, of a 40,000-particle state-based bar
+// 84 against 484 us.  16 warps of 128 registers on an SM; 24 warps of 80
+// (spills) were slower, 592 against 474 us per step of a 64^3 cube.
+// ---------------------------------------------------------------------
+// Largest family evaluated in shared memory: 288 slots of 768 bytes and
+// their broken bits, within the 227 KB a block may take.
+constexpr int32_t kForceSlots = 288;
+constexpr int64_t kWideSlices = 148;  // SMs of a B200
+inline size_t force_slice_bytes(int32_t cap) { return 768 * (size_t)cap + 128 * (size_t)((cap + 31) / 32); }
+
+// A bond the branch-free evaluation does not cover, with the operators.
+template <int KIND>
+__device__ __noinline__ bool bond_term_general(const Geo &g, const DevBlock &B, int64_t p, int tp, int32_t q,
+                                               const double4 *__restrict__ y, const double2 *__restrict__ mth,
+                                               double *t) {
+    return bond_term<KIND>(g, B, tp, g.x4[p], y[p], KIND != PD_MAT_BOND_BASED ? mth[p] : make_double2(0.0, 0.0),
+                           g.tdens[B.type_base + tp], q, y, mth, t[0], t[1], t[2]);
+}
+
+// A particle of a slice the block evaluation does not cover (accumulating).
+__device__ __noinline__ void force_particle_general(const Geo &g, int64_t p, int32_t ti, int kind,
+                                                    const double4 *__restrict__ y, const double2 *__restrict__ mth,
+                                                    const uint32_t *__restrict__ win, uint32_t *__restrict__ wout,
+                                                    double4 *__restrict__ f) {
+    if (kind == PD_MAT_BOND_BASED) force_serial_particle<PD_MAT_BOND_BASED>(g, p, ti, y, mth, win, wout, f, 1);
+    else force_serial_particle<PD_MAT_ORDINARY_STATE_BASED>(g, p, ti, y, mth, win, wout, f, 1);
+}
+
+// What a slot's evaluation needs of its neighbour.
+struct SlotIn {
+    double4 x, y;
+    double2 m;
+    int32_t q;
+};
+
+template <int KIND, bool MULTI, bool ST, int NW>
+__device__ __forceinline__ void evaluate_slice(const Geo &g, const DevBlock &B, const SliceInfo &d, int64_t p,
+                                               int32_t ti, int32_t n, int32_t L, int w, int lane,
+                                               const double4 *__restrict__ y, const double2 *__restrict__ mth,
+                                               const uint32_t *__restrict__ win, double *term, uint32_t *brk) {
+    constexpr bool PMB = KIND == PD_MAT_BOND_BASED;
+    const int tp = ti >= 0 ? ti & 255 : 0;
+    const double4 xp = ld4(g.x4 + p), yp = ld4(y + p);
+    const double2 mp = PMB ? make_double2(0.0, 0.0) : mth[p];
+    const double rho_p = g.tdens[B.type_base + tp];
+    const PairParam pp0 = g.pairs[B.pair_base + tp + tp * B.nt];
+    const double c11 = B.c11;
+    const bool own_ok = div_ok(rho_p) && (PMB ? div_ok(fabs(c11)) : div_ok(mp.x));
+    const double rrho = rcp_rn(rho_p), rmp = PMB ? 0.0 : rcp_rn(mp.x);
+    const int32_t *nb = g.nbr + d.nbr + (ST ? 0 : lane);
+    const uint32_t *wi = win + d.word + lane;
+    // warp w evaluates the contiguous slots [k0, k1)
+    const int32_t per = (L + NW - 1) / NW, k0 = min(w * per, L), k1 = min(k0 + per, L);
+    if (k0 >= k1) return;
+    // (a stencil offset is in range for every lane with bonds)
+    const int32_t some = n > 0 ? -1 : 0;
+    auto neighbour = [&](int32_t k) -> int32_t {
+        if (ST) return (int32_t)p + (__ldg(nb + k) & some);
+        return k < n ? __ldg(nb + 32 * k) : (int32_t)p;
+    };
+    auto load = [&](int32_t q) {
+        SlotIn r;
+        r.x = ld4(g.x4 + q);
+        r.y = ld4(y + q);
+        r.m = PMB ? make_double2(0.0, 0.0) : __ldg(mth + q);
+        r.q = q;
+        return r;
+    };
+    // The slot's term (zero unless live and within the critical stretch);
+    // returns whether the evaluation is exact.  The numerators: ext is zero
+    // or at least 2^-54 of the lengths, and so is s, at most 2^200; PMB: c in
+    // [2^-100, 2^100) then keeps 0.5 t in range, LPS checks it; V < 2^100
+    // bounds the last three from above.
+    auto evaluate = [&](const SlotIn &r, bool live, double &o0, double &o1, double &o2, bool &within) -> bool {
+        const double Y1 = r.y.x - yp.x, Y2 = r.y.y - yp.y, Y3 = r.y.z - yp.z;
+        const double X1 = r.x.x - xp.x, X2 = r.x.y - xp.y, X3 = r.x.z - xp.z;
+        double xij, yij, rx, ry;
+        bool fast = sqrt_rcp_rn(X1 * X1 + X2 * X2 + X3 * X3, xij, rx) && own_ok;
+        fast = sqrt_rcp_rn(Y1 * Y1 + Y2 * Y2 + Y3 * Y3, yij, ry) && fast;
+        fast = (uint32_t)hi_word(r.x.w) < ((1023u + 100u) << 20) && fast;
+        const PairParam pp = MULTI ? g.pairs[B.pair_base + tp + (g.tinfo[r.q] & 255) * B.nt] : pp0;
+        const double ext = yij - xij;
+        const double s = div_rn(ext, xij, rx);
+        within = s < pp.cs;
+        double t;
+        if (PMB) {
+            t = s * c11;
+        } else {
+            fast = fast && div_ok(r.m.x);
+            const double a = div_rn(rx, mp.x, rmp), b = div_rn(rx, r.m.x, rcp_rn(r.m.x));
+            t = pp.k35 * (mp.y * xij * a + r.m.y * xij * b) + pp.g15 * ext * (a + b);
+        }
+        const double ht = 0.5 * t;
+        if (!PMB) fast = fast && magnitude(ht) >= kMagLo && (2u * (uint32_t)hi_word(ht)) < kMagHi;
+        double xx = div_rn(ht, yij, ry);
+        xx = live && within ? xx : 0.0;
+        o0 = xx * Y1 * r.x.w;
+        o1 = xx * Y2 * r.x.w;
+        o2 = xx * Y3 * r.x.w;
+        fast = fast && min(min(magnitude(o0), magnitude(o1)), magnitude(o2)) >= kMagLo;
+        o0 = div_rn(o0, rho_p, rrho);
+        o1 = div_rn(o1, rho_p, rrho);
+        o2 = div_rn(o2, rho_p, rrho);
+        return fast;
+    };
+    uint32_t bits = 0, gone = 0;
+    auto finish = [&](int32_t k, int32_t q, bool live, bool exact, bool within, double o0, double o1, double o2) {
+        if (live && !exact) {
+            double out[3] = {0.0, 0.0, 0.0};
+            within = bond_term_general<KIND>(g, B, p, tp, q, y, mth, out);
+            o0 = out[0];
+            o1 = out[1];
+            o2 = out[2];
+        }
+        if (live && !within) gone |= 1u << (k & 31);
+        double *t = term + 96 * k + lane;
+        t[0] = live ? o0 : 0.0;
+        t[32] = live ? o1 : 0.0;
+        t[64] = live ? o2 : 0.0;
+    };
+    // two slots at a time, their chains side by side (a chain is some 35
+    // dependent FP64 operations of 16 cycles, and 16 warps fit an SM)
+    int32_t qa = neighbour(k0), qb = neighbour(min(k0 + 1, k1 - 1));
+    for (int32_t k = k0; k < k1;) {
+        const int32_t word = k >> 5, kw = min(k1, (word + 1) << 5);  // slots of one intact word
+        bits = 32 * word < n ? wi[32 * word] : 0u;
+        gone = 0;
+        for (; k < kw; k += 2) {
+            const bool two = k + 1 < kw;
+            const SlotIn ra = load(qa), rb = load(two ? qb : qa);
+            const int32_t next = two ? k + 2 : k + 1;
+            qa = neighbour(min(next, k1 - 1));
+            qb = neighbour(min(next + 1, k1 - 1));
+            const uint32_t b2 = bits >> (k & 31);
+            const bool la = (b2 & 1u) != 0u, lb = (b2 & 2u) != 0u;
+            double a0, a1, a2, b0, b1, bz;
+            bool wa, wb;
+            const bool ea = evaluate(ra, la, a0, a1, a2, wa), eb = evaluate(rb, lb, b0, b1, bz, wb);
+            finish(k, ra.q, la, ea, wa, a0, a1, a2);
+            if (two) finish(k + 1, rb.q, lb, eb, wb, b0, b1, bz);
+        }
+        k = kw;
+        if (gone) atomicOr(brk + 32 * word + lane, gone);  // two warps may own parts of one word
+    }
+}
+
+template <int KIND, int NW>
+__device__ __forceinline__ void evaluate_kind(const Geo &g, const DevBlock &B, const SliceInfo &d, int64_t p,
+                                              int32_t ti, int32_t n, int32_t L, int w, int lane,
+                                              const double4 *__restrict__ y, const double2 *__restrict__ mth,
+                                              const uint32_t *__restrict__ win, double *term, uint32_t *brk) {
+    if (d.mode == kStencil) {
+        if (B.nt > 1) evaluate_slice<KIND, true, true, NW>(g, B, d, p, ti, n, L, w, lane, y, mth, win, term, brk);
+        else evaluate_slice<KIND, false, true, NW>(g, B, d, p, ti, n, L, w, lane, y, mth, win, term, brk);
+    } else {
+        if (B.nt > 1) evaluate_slice<KIND, true, false, NW>(g, B, d, p, ti, n, L, w, lane, y, mth, win, term, brk);
+        else evaluate_slice<KIND, false, false, NW>(g, B, d, p, ti, n, L, w, lane, y, mth, win, term, brk);
+    }
+}
+
+template <int NW>
+__global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 1)
+    k_force_slice(Geo g, const double4 *__restrict__ y, const double2 *__restrict__ mth,
+                  const uint32_t *__restrict__ win, uint32_t *__restrict__ wout, double4 *__restrict__ f,
+                  int accumulate, int32_t cap, int64_t s0) {
+    extern __shared__ double term[];  // [slot][component][lane], then the broken bits [word][lane]
+    const int64_t s = s0 + blockIdx.x;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t p = 32 * s + lane;
+    const int32_t ti = g.tinfo[p], n = g.cnt[p];
+    const SliceInfo d = g.si[s];
+    const int32_t L = slice_slots(n);
+    // every particle of a slice belongs to one block (padding: -1)
+    const int32_t tb = __reduce_max_sync(0xffffffffu, ti);
+    const int kind = tb >= 0 ? g.blocks[tb >> 8].kind : PD_MAT_SKIP;
+    if (kind == PD_MAT_ELASTO_PLASTIC || L > cap) return;
+    const int32_t words = (L + 31) >> 5;
+    uint32_t *brk = reinterpret_cast<uint32_t *>(term + 96 * (int64_t)cap);
+    const uint32_t *wi = win + d.word + lane;
+    uint32_t *wo = wout + d.word + lane;
+    if (kind == PD_MAT_SKIP || g.deformed[tb >> 8] == 0) {
+        for (int32_t c = w; c < words; c += NW)
+            if (32 * c < n) wo[32 * c] = wi[32 * c];
+        if (w == 0 && !accumulate) f[p] = make_double4(0.0, 0.0, 0.0, 0.0);
+        return;
+    }
+    if (accumulate) {
+        const double4 f0 = f[p];
+        const uint64_t nz = 0x8000000000000000ull;
+        const bool neg = (uint64_t)__double_as_longlong(f0.x) == nz || (uint64_t)__double_as_longlong(f0.y) == nz ||
+                         (uint64_t)__double_as_longlong(f0.z) == nz;
+        if (__any_sync(0xffffffffu, neg)) {  // the same lanes in every warp
+            if (w == 0 && ti >= 0) force_particle_general(g, p, ti, kind, y, mth, win, wout, f);
+            return;
+        }
+    }
+    for (int32_t c = w; c < words; c += NW) brk[32 * c + lane] = 0u;
+    __syncthreads();
+    const DevBlock &B = g.blocks[tb >> 8];
+    if (kind == PD_MAT_BOND_BASED)
+        evaluate_kind<PD_MAT_BOND_BASED, NW>(g, B, d, p, ti, n, L, w, lane, y, mth, win, term, brk);
+    else
+        evaluate_kind<PD_MAT_ORDINARY_STATE_BASED, NW>(g, B, d, p, ti, n, L, w, lane, y, mth, win, term, brk);
+    __syncthreads();
+    if (w >= 3) {
+        for (int32_t c = w - 3; c < words; c += NW - 3)
+            if (32 * c < n) wo[32 * c] = wi[32 * c] & ~brk[32 * c + lane];
+        return;
+    }
+    // kp: slots with q > p (a prefix: slots descend in q)
+    int32_t lo = 0, hi = n;
+    {
+        const bool st = d.mode == kStencil;
+        const int32_t *nb = g.nbr + d.nbr + (st ? 0 : lane);
+        const int32_t own = st ? 0 : (int32_t)p;
+        while (lo < hi) {
+            const int32_t mid = (lo + hi) >> 1;
+            if ((st ? nb[mid] : nb[32 * mid]) > own) lo = mid + 1;
+            else hi = mid;
+        }
+    }
+    const int32_t kp = lo;
+    const int32_t kmin = (int32_t)__reduce_min_sync(0xffffffffu, (unsigned)(n > 0 ? kp : L));
+    const int32_t kmax = (int32_t)__reduce_max_sync(0xffffffffu, (unsigned)kp);
+    const double *T = term + 32 * w + lane;
+    double *fo = reinterpret_cast<double *>(f + p);
+    double a = accumulate ? fo[w] : 0.0;
+#pragma unroll 8
+    for (int32_t k = L - 1; k >= kmin; --k) {
+        const double t = T[96 * k];
+        a = a + (k >= kp ? t : 0.0);
+    }
+#pragma unroll 8
+    for (int32_t k = 0; k < L; ++k) a = a + T[96 * k];
+#pragma unroll 8
+    for (int32_t k = kmax - 1; k >= 0; --k) {
+        const double t = T[96 * k];
+        a = a + (k < kp ? t : 0.0);
+    }
+    if (ti >= 0) {
+        fo[w] = a;
+        if (w == 0) fo[3] = 0.0;
+    } else if (!accumulate) {
+        fo[w] = 0.0;
+        if (w == 0) fo[3] = 0.0;
+    }
 }
 
 // ---------------------------------------------------------------------
@@ -949,10 +1276,19 @@ void launch_weighted_volume(cudaStream_t st, const Geo &g, double2 *mth) {
     k_weighted_volume<<<grid_for(g.N), kThreads, 0, st>>>(g, mth); pd::note_launch();
 }
 
+// Sixteen warps per slice when every slice has an SM to itself, else eight:
+// a 990-particle cube 26.9 against 28.3 us per step with eight, a
+// 40,000-particle bar (two blocks of eight on an SM, one of sixteen) 177
+// against 144 us.
+static bool wide_slices(int64_t slices) { return slices <= kWideSlices; }
+
 void launch_theta_serial(cudaStream_t st, const Geo &g, const double4 *y, const uint32_t *win,
                          double2 *mth, int64_t p0, int64_t p1) {
     if (p1 <= p0) return;
-    k_theta_serial<<<grid_for(p1 - p0), kThreads, 0, st>>>(g, y, win, mth, p0, p1); pd::note_launch();
+    const int64_t S = (p1 - p0) / 32;
+    if (wide_slices(S)) k_theta_slice<16><<<(unsigned)S, 512, 0, st>>>(g, y, win, mth, p0 / 32);
+    else k_theta_slice<8><<<(unsigned)S, 256, 0, st>>>(g, y, win, mth, p0 / 32);
+    pd::note_launch();
 }
 
 void launch_td_serial(cudaStream_t st, const Geo &g, const double4 *y, const double2 *mth,
@@ -962,12 +1298,36 @@ void launch_td_serial(cudaStream_t st, const Geo &g, const double4 *y, const dou
     pd::note_launch();
 }
 
+// k_force_slice may use more than the default 48 KB of shared memory; the
+// limit is a setting per kernel and device, made once (with the device
+// current).
+static void force_slice_attrs() {
+    static std::atomic<bool> done[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || done[dev].load()) return;
+    const int bytes = (int)force_slice_bytes(kForceSlots);
+    if (cudaFuncSetAttribute(k_force_slice<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess &&
+        cudaFuncSetAttribute(k_force_slice<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess)
+        done[dev].store(true);
+}
+
 void launch_force_serial(cudaStream_t st, const Geo &g, const double4 *y, const double2 *mth,
                          const uint32_t *win, uint32_t *wout, double4 *f, int accumulate,
                          int64_t p0, int64_t p1) {
     if (p1 <= p0) return;
-    k_force_serial<<<grid_for(p1 - p0), kThreads, 0, st>>>(g, y, mth, win, wout, f, accumulate,
-                                                           p0, p1); pd::note_launch();
+    const int32_t cap = g.max_slots < kForceSlots ? g.max_slots : kForceSlots;
+    const size_t sm = force_slice_bytes(cap);
+    const int64_t S = (p1 - p0) / 32;
+    force_slice_attrs();
+    if (wide_slices(S))
+        k_force_slice<16><<<(unsigned)S, 512, sm, st>>>(g, y, mth, win, wout, f, accumulate, cap, p0 / 32);
+    else
+        k_force_slice<8><<<(unsigned)S, 256, sm, st>>>(g, y, mth, win, wout, f, accumulate, cap, p0 / 32);
+    pd::note_launch();
+    if (g.has_ep || g.max_slots > cap) {
+        k_force_serial<<<grid_for(p1 - p0), kThreads, 0, st>>>(g, y, mth, win, wout, f, accumulate, cap, p0, p1);
+        pd::note_launch();
+    }
 }
 
 void launch_kick_drift(cudaStream_t st, int64_t N, double c, double dt, const double4 *f,

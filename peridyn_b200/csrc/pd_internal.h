@@ -117,6 +117,8 @@ struct Geo {
     const int32_t *nbr;        // bond index data (see SliceInfo)
     const uint32_t *fam;       // family-member bits (same layout as intact)
     const int32_t *deformed;   // per block
+    int32_t max_slots;         // largest slot count of a particle
+    int32_t has_ep;            // some block is elasto-plastic
     // elasto-plastic blocks: td_norm2 per particle, plastic deviatoric
     // strain per bond slot (read from edp_in, written to edp_out)
     double *td2;
