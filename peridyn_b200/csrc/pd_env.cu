@@ -84,6 +84,7 @@ pd::Geo pd_env::geo() const {
     g.nbr = nbr.p;
     g.fam = fam.p;
     g.deformed = deformed.p;
+    g.stop = nullptr;
     g.max_slots = max_slots;
     g.has_ep = 0;
     for (const auto &b : hb)
@@ -1140,6 +1141,31 @@ extern "C" pd_status pd_env_finalize(pd_env *env) {
             d.sn = (int64_t)sidx.size();
         }
         env->bcs.push_back(std::move(d));
+    }
+    // membership bits and list places for the serial mode's fused integration
+    if (env->precision == PD_PREC_FP64_SERIAL && !env->hbc.empty() && env->hbc.size() <= (size_t)kMaxFusedBC) {
+        std::vector<uint8_t> bits(N, 0);
+        std::vector<int32_t> rank;
+        for (size_t k = 0; k < env->hbc.size(); ++k) {
+            const auto &ei = env->hbc[k].env_idx;
+            const int64_t lo = ei.empty() ? 0 : env->map_h[ei.front()];
+            const size_t base = rank.size();
+            env->bc_rank_lo.push_back(lo);
+            env->bc_rank_off.push_back((int64_t)base);
+            if (ei.empty()) continue;
+            rank.resize(base + (size_t)(env->map_h[ei.back()] - lo + 1), -1);
+            for (size_t r = 0; r < ei.size(); ++r) {
+                const int64_t q = env->map_h[ei[r]];
+                rank[base + (size_t)(q - lo)] = (int32_t)r;
+                bits[q] |= (uint8_t)(1u << k);
+            }
+        }
+        PD_TRY(env->bc_bits.alloc(N));
+        PD_TRY(env->bc_rank.alloc(std::max<size_t>(rank.size(), 1)));
+        CK(cudaMemcpyAsync(env->bc_bits.p, bits.data(), N, cudaMemcpyHostToDevice, st));
+        if (!rank.empty())
+            CK(cudaMemcpyAsync(env->bc_rank.p, rank.data(), rank.size() * 4, cudaMemcpyHostToDevice, st));
+        CK(cudaStreamSynchronize(st));
     }
     PD_TRY(pd::contacts_finalize(env));
     CK(cudaStreamSynchronize(st));

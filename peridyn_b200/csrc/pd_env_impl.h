@@ -235,6 +235,11 @@ struct pd_env {
     std::vector<int> deformed0;  // gate flags right after finalize
     pd::DBuf<int32_t> flag;
     std::vector<pd::DevBC> bcs;
+    // serial mode, up to kMaxFusedBC conditions: membership bits and places
+    // in the conditions' lists (FusedBCs)
+    pd::DBuf<uint8_t> bc_bits;
+    pd::DBuf<int32_t> bc_rank;
+    std::vector<int64_t> bc_rank_off, bc_rank_lo;
     std::vector<pd::DevContact> contacts;
     int64_t contact_epoch = 0;  // incremented whenever the contact lists change
 
@@ -244,6 +249,7 @@ struct pd_env {
     pd::DBuf<int32_t> scr_i;   // per-particle count scratch (bond counts)
     pd::DBuf<int32_t> free_mask;
     pd::DBuf<double> red;
+    pd::DBuf<int32_t> qs_state;  // QsState of pd_env_qsdrag
 
     // optional CUDA-event timing of the bond-force kernel launches
     bool prof = false;
@@ -301,5 +307,6 @@ pd_status fast_land_flags(pd_env *env);
 // estimate from particle counts and family rows; for admission control).
 int64_t footprint_estimate(const pd_env *env);
 pd_status fast_update_acc(pd_env *env);
-pd_status update_acc_serial(pd_env *env);
+// momentum: p = m v at the end; stop: see Geo::stop.
+pd_status update_acc_serial(pd_env *env, bool momentum = true, const int32_t *stop = nullptr);
 }  // namespace pd

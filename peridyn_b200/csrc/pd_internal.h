@@ -119,6 +119,7 @@ struct Geo {
     const int32_t *deformed;   // per block
     int32_t max_slots;         // largest slot count of a particle
     int32_t has_ep;            // some block is elasto-plastic
+    const int32_t *stop;       // not null: the force kernels return at once when *stop is set
     // elasto-plastic blocks: td_norm2 per particle, plastic deviatoric
     // strain per bond slot (read from edp_in, written to edp_out)
     double *td2;
@@ -209,6 +210,28 @@ void launch_force_serial(cudaStream_t st, const Geo &g, const double4 *y, const 
 // elasto_plastic.jl:166-172 out_of_loop! td_norm2 pass (breaks bonds too)
 void launch_td_serial(cudaStream_t st, const Geo &g, const double4 *y, const double2 *mth,
                       const uint32_t *win, uint32_t *wout, int64_t p0, int64_t p1);
+
+// Boundary conditions of the fused integration kernel: at most
+// kMaxFusedBC, each with the directions of the velocity and position
+// conditions and, for every particle p of its index range, the place of p in
+// its list (rank[p - lo]).
+constexpr int kMaxFusedBC = 8;
+struct FusedBC {
+    BCDev bc;
+    int64_t lo;
+    const int32_t *rank;
+    int32_t dir_vel, dir_pos;
+};
+struct FusedBCs {
+    int32_t n;
+    const uint8_t *bits;  // bit k: the particle belongs to condition k
+    FusedBC c[kMaxFusedBC];
+};
+// post: the second half of a step (p = m v when p is not null, half kick,
+// velocity conditions); pre: the first half of the next (half kick, drift,
+// position conditions at time step ts).
+void launch_advance(cudaStream_t st, int64_t N, double c, double dt, bool post, bool pre, const double4 *f,
+                    double4 *v, double4 *y, const double *mass, double4 *p, const FusedBCs &bcs, int64_t ts);
 
 // Elementwise velocity-Verlet pieces (exact FP64 arithmetic).
 void launch_kick_drift(cudaStream_t st, int64_t N, double c, double dt, const double4 *f,

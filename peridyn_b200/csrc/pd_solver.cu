@@ -123,13 +123,24 @@ constexpr int kRedBlocks = 148;
 // (fixed for the same reason).
 constexpr int kGateWidth = 148;
 
+// Progress of a quasi-static minimisation on the device.
+struct QsState {
+    double h[2];      // max|f|, max|dy| of the last iteration
+    int64_t iters;    // iterations applied
+    int32_t done;     // both below their tolerances: later iterations do nothing
+    uint32_t arrived;
+};
+
 // minimize.jl:149-155 apply_! and :202 y[:, mask] .+= dy, fused with the
-// max|f| / max|dy| reductions of :204.
+// max|f| / max|dy| reductions of :204 and the convergence test: the last
+// block to arrive combines the blocks' maxima (exact in any order).
 __global__ void __launch_bounds__(256)
     k_qs_apply(int64_t N, const int32_t *__restrict__ freem, const double4 *__restrict__ f,
                double4 *__restrict__ opt, double4 *__restrict__ y, double lambda, double kk,
-               double ss, double a, double *__restrict__ partial) {
+               double ss, double a, double f_tol, double x_tol, double *__restrict__ partial, QsState *qs) {
     __shared__ double sf[256], sy[256];
+    __shared__ bool last;
+    if (*(volatile int32_t *)&qs->done) return;
     double mf = 0.0, my = 0.0;
     for (int64_t i = blockIdx.x * 256 + threadIdx.x; i < N; i += (int64_t)kRedBlocks * 256) {
         if (!freem[i]) continue;
@@ -147,30 +158,38 @@ __global__ void __launch_bounds__(256)
         opt[i] = make_double4(o[0], o[1], o[2], 0.0);
         y[i] = make_double4(yy[0], yy[1], yy[2], yi.w);
     }
-    sf[threadIdx.x] = mf;
-    sy[threadIdx.x] = my;
-    __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if (threadIdx.x < s) {
-            sf[threadIdx.x] = nanmax(sf[threadIdx.x], sf[threadIdx.x + s]);
-            sy[threadIdx.x] = nanmax(sy[threadIdx.x], sy[threadIdx.x + s]);
-        }
+    auto reduce = [&](double vf, double vy) {
+        sf[threadIdx.x] = vf;
+        sy[threadIdx.x] = vy;
         __syncthreads();
-    }
+        for (int s = 128; s > 0; s >>= 1) {
+            if (threadIdx.x < s) {
+                sf[threadIdx.x] = nanmax(sf[threadIdx.x], sf[threadIdx.x + s]);
+                sy[threadIdx.x] = nanmax(sy[threadIdx.x], sy[threadIdx.x + s]);
+            }
+            __syncthreads();
+        }
+    };
+    reduce(mf, my);
     if (threadIdx.x == 0) {
         partial[2 * blockIdx.x] = sf[0];
         partial[2 * blockIdx.x + 1] = sy[0];
+        __threadfence();
+        last = atomicAdd(&qs->arrived, 1u) == gridDim.x - 1;
     }
-}
-
-__global__ void k_qs_final(const double *__restrict__ partial, double *__restrict__ out2) {
-    double mf = 0.0, my = 0.0;
-    for (int b = 0; b < kRedBlocks; ++b) {
-        mf = nanmax(mf, partial[2 * b]);
-        my = nanmax(my, partial[2 * b + 1]);
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const bool one = threadIdx.x < kRedBlocks;
+    const volatile double *vp = partial;
+    reduce(one ? vp[2 * threadIdx.x] : 0.0, one ? vp[2 * threadIdx.x + 1] : 0.0);
+    if (threadIdx.x == 0) {
+        qs->h[0] = sf[0];
+        qs->h[1] = sy[0];
+        qs->iters += 1;
+        qs->arrived = 0;
+        if (sf[0] < f_tol && sy[0] < x_tol) qs->done = 1;
     }
-    out2[0] = mf;
-    out2[1] = my;
 }
 
 __global__ void k_set_free(int64_t N, const int32_t *__restrict__ tinfo, int32_t *__restrict__ freem) {
@@ -190,9 +209,10 @@ __global__ void k_clear_idx(int64_t n, const int32_t *__restrict__ idx, int32_t 
 namespace pd {
 
 // update_acc! (solvers.jl:320-336) in serial-order FP64.
-pd_status update_acc_serial(pd_env *env) {
+pd_status update_acc_serial(pd_env *env, bool momentum, const int32_t *stop) {
     cudaStream_t st = env->st;
     Geo g = env->geo();
+    g.stop = stop;
     // force_density! gate for blocks still undeformed
     std::vector<GateItem> items;
     for (size_t b = 0; b < env->hb.size() && !env->gate_hold; ++b) {
@@ -243,7 +263,7 @@ pd_status update_acc_serial(pd_env *env) {
     // short_range_contact!
     PD_TRY(contacts_force(env));
     // update_misc!
-    launch_momentum(st, env->N, env->mass.p, env->v.p, env->p.p);
+    if (momentum) launch_momentum(st, env->N, env->mass.p, env->v.p, env->p.p);
     CK(cudaGetLastError());
     return PD_OK;
 }
@@ -285,21 +305,62 @@ extern "C" pd_status pd_env_apply_bc_at0(pd_env *env) {
     return PD_OK;
 }
 
+// The fused integration's view of the conditions: the directions of the
+// velocity conditions as they are now, of the position conditions filled in
+// by the caller.
+static FusedBCs fused_bcs(pd_env *env) {
+    FusedBCs b;
+    std::memset(&b, 0, sizeof(b));
+    b.n = (int32_t)env->hbc.size();
+    b.bits = env->bc_bits.p;
+    for (size_t k = 0; k < env->hbc.size(); ++k) {
+        b.c[k].bc = bc_view(env, k);
+        b.c[k].lo = env->bc_rank_lo[k];
+        b.c[k].rank = env->bc_rank.p + env->bc_rank_off[k];
+        b.c[k].dir_vel = b.c[k].dir_pos = env->hbc[k].dir;
+    }
+    return b;
+}
+
 // velocity_verlet.jl:57-89, nsteps times, in the serial mode, enqueued on
-// the environment's stream.
+// the environment's stream.  With at most kMaxFusedBC conditions the second
+// half of a step and the first half of the next run as one kernel.
 static pd_status serial_steps(pd_env *env, int64_t nsteps) {
     const double c = env->dt / 2;
     const double dt = env->dt;
+    const bool fused = env->hbc.size() <= (size_t)kMaxFusedBC;
+    FusedBCs b;
+    auto advance = [&](bool post, bool pre, double4 *p) {
+        launch_advance(env->st, env->N, c, dt, post, pre, env->f.p, env->v.p, env->y.p, env->mass.p, p, b, env->ts);
+    };
+    if (fused && nsteps > 0) {
+        b = fused_bcs(env);
+        advance(false, true, nullptr);
+    }
     for (int64_t s = 0; s < nsteps; ++s) {
-        launch_kick_drift(env->st, env->N, c, dt, env->f.p, env->v.p, env->y.p);
-        for (size_t k = 0; k < env->hbc.size(); ++k)
-            launch_bc_pos(env->st, bc_view(env, k), dt, env->hbc[k].dir, env->ts, env->y.p);
-        PD_TRY(update_acc_serial(env));
-        launch_kick(env->st, env->N, c, env->f.p, env->v.p);
-        for (size_t k = 0; k < env->hbc.size(); ++k)
-            launch_bc_vel(env->st, bc_view(env, k), env->hbc[k].dir, env->y.p, env->v.p);
-        bc_check(env);
-        env->ts += 1;
+        const bool last = s == nsteps - 1;
+        if (!fused) {
+            launch_kick_drift(env->st, env->N, c, dt, env->f.p, env->v.p, env->y.p);
+            for (size_t k = 0; k < env->hbc.size(); ++k)
+                launch_bc_pos(env->st, bc_view(env, k), dt, env->hbc[k].dir, env->ts, env->y.p);
+        }
+        PD_TRY(update_acc_serial(env, !fused));
+        if (fused) {
+            bool scales = false;  // ScaleFixWait's check! moves particles between the two halves
+            for (const auto &h : env->hbc) scales |= h.scales_at(env->ts);
+            b = fused_bcs(env);
+            if (last || scales) advance(true, false, last ? env->p.p : nullptr);
+            bc_check(env);
+            env->ts += 1;
+            for (size_t k = 0; k < env->hbc.size(); ++k) b.c[k].dir_pos = env->hbc[k].dir;
+            if (!last) advance(!scales, true, nullptr);
+        } else {
+            launch_kick(env->st, env->N, c, env->f.p, env->v.p);
+            for (size_t k = 0; k < env->hbc.size(); ++k)
+                launch_bc_vel(env->st, bc_view(env, k), env->hbc[k].dir, env->y.p, env->v.p);
+            bc_check(env);
+            env->ts += 1;
+        }
         if ((s & 63) == 63) CK(cudaGetLastError());
     }
     CK(cudaGetLastError());
@@ -355,7 +416,8 @@ extern "C" pd_status pd_env_qsdrag(pd_env *env, double step_size, double drag, i
     // :138-145 free particles: not in any BC that acts beyond the start
     if (!env->free_mask.p) PD_TRY(env->free_mask.alloc(N));
     if (!env->opt.p) PD_TRY(env->opt.alloc(N));
-    if (!env->red.p) PD_TRY(env->red.alloc(2 * kRedBlocks + 2));
+    if (!env->red.p) PD_TRY(env->red.alloc(2 * kRedBlocks));
+    if (!env->qs_state.p) PD_TRY(env->qs_state.alloc((sizeof(QsState) + 3) / 4));
     k_set_free<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(N, env->tinfo.p, env->free_mask.p); pd::note_launch();
     for (size_t k = 0; k < env->hbc.size(); ++k)
         if (!env->hbc[k].onlyatstart && env->bcs[k].n > 0)
@@ -366,19 +428,39 @@ extern "C" pd_status pd_env_qsdrag(pd_env *env, double step_size, double drag, i
     const double lambda = drag;
     const double kk = lambda / 10;
     const double a = ps / 10;
-    int64_t it = 0;
-    for (int64_t i = 1; i <= max_iter; ++i) {
-        it = i;
-        PD_TRY(update_acc_serial(env));
-        k_qs_apply<<<kRedBlocks, 256, 0, st>>>(N, env->free_mask.p, env->f.p, env->opt.p, env->y.p, lambda, kk,
-                                               step_size, a, env->red.p); pd::note_launch();
-        k_qs_final<<<1, 1, 0, st>>>(env->red.p, env->red.p + 2 * kRedBlocks); pd::note_launch();
+    // Iterations are enqueued in batches of up to kQsBatch between two reads
+    // of the progress; an iteration after the converged one finds the done
+    // flag and changes nothing (a read-back per iteration cost 10 us of 70 on
+    // a 9,500-particle bar).  While a block is undeformed, or with contacts,
+    // whose kernels do not look at the flag, every iteration is read.
+    constexpr int64_t kQsBatch = 16;
+    QsState *qs = (QsState *)env->qs_state.p;
+    CK(cudaMemsetAsync(qs, 0, sizeof(QsState), st));
+    QsState h{};
+    const bool ep = env->geo().has_ep != 0;
+    for (int64_t batch = 2; h.iters < max_iter && !h.done; batch = std::min(2 * batch, kQsBatch)) {
+        PD_TRY(refresh_deformed(env));
+        bool known = env->hc.empty();
+        for (size_t b = 0; b < env->hb.size() && !env->gate_hold; ++b)
+            if (env->hb[b].kind != PD_MAT_SKIP && !env->deformed_h[b]) known = false;
+        const int64_t m = known ? std::min(batch, max_iter - h.iters) : 1;
+        const int64_t it0 = h.iters;
+        const int cur0 = env->cur, ecur0 = env->ecur;
+        for (int64_t i = 0; i < m; ++i) {
+            PD_TRY(update_acc_serial(env, false, &qs->done));
+            k_qs_apply<<<kRedBlocks, 256, 0, st>>>(N, env->free_mask.p, env->f.p, env->opt.p, env->y.p, lambda, kk,
+                                                   step_size, a, f_tol, x_tol, env->red.p, qs); pd::note_launch();
+        }
         CK(cudaGetLastError());
-        double h[2];
-        CK(cudaMemcpyAsync(h, env->red.p + 2 * kRedBlocks, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(&h, qs, sizeof(h), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        if ((h[0] < f_tol) && (h[1] < x_tol)) break;
+        // the buffers as the iterations that ran left them
+        const int odd = (int)((h.iters - it0) & 1);
+        env->cur = ep ? cur0 : cur0 ^ odd;
+        env->ecur = ep ? ecur0 ^ odd : ecur0;
     }
+    const int64_t it = h.iters;
+    launch_momentum(st, N, env->mass.p, env->v.p, env->p.p);
     (void)dt;
     bc_check(env);
     env->ts += 1;

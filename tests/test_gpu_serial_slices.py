@@ -98,3 +98,68 @@ def test_accumulating_into_negative_zeros(oracle, law):
     assert np.array_equal(f, ora.f)
     assert np.array_equal(np.signbit(f), np.signbit(ora.f))
     env.close()
+
+
+@pytest.mark.parametrize("conditions", [1, 4, 9])  # fused integration: at most 8
+def test_several_conditions_on_the_same_particles(oracle, conditions):
+    m = _body("lps", (14, 6, 5), 3.015)
+    x = m.general.x
+    lo, hi = x[0].min(), x[0].max()
+    bcs = [pb.FixBC(x[0] < lo + 2.0e-3, dims=(True, False, True)),
+           pb.ToFroBC(x[0] > hi - 2.0e-3, [0.5, 0.0, -0.25], 5.0, applyafter=3),
+           pb.ContainerBC(x[1] < x[1].mean(), limits=None),
+           pb.ContainerBC(x[0] > lo + 5.0e-3, limits=np.array([[lo, hi], [x[1].min(), x[1].max()],
+                                                               [x[2].min(), x[2].max()]]))]
+    bcs += [pb.FixBC((x[0] < lo + 1.5e-3) & (x[1] < x[1].min() + k * 1.0e-3), dims=(False, True, False))
+            for k in range(1, 6)]
+    bcs = bcs[:conditions]
+    env = pb.Env(1, [m], [], bcs, 2.0e-8)
+    ora = oracle.OracleEnv([m], [], bcs, 2.0e-8)
+    ora.apply_bc_at0()
+    pb.apply_bc_at0(env, 0)
+    for n in (1, 9, 6):
+        pb.velocity_verlet_step(env, nsteps=n)
+        for _ in range(n):
+            ora.vv_step()
+    _same(env, ora)
+    assert np.array_equal(env.p, ora.p)
+    env.close()
+
+
+@pytest.mark.parametrize("max_iter,f_tol", [(1, 1e-3), (2, 1e-3), (3, 1e-3), (7, 1e-3), (40, 1e-3), (40, 1e30),
+                                            (40, "fifth")])
+def test_minimize_stops_where_the_loop_does(oracle, max_iter, f_tol):
+    """Iterations run in batches between two reads of the progress; the state
+    is the one of the iteration that converged."""
+    def build():
+        m = _body("lps", (11, 5, 5), 3.015, jitter=0.0)
+        x = m.general.x
+        m.general.velocity[:] = 0.0
+        bcs = [pb.FixBC(x[0] < x[0].min() + 1.5e-3), pb.MoveBC(x[0] > x[0].max() - 1.5e-3, [10.0, 0.0, 0.0])]
+        return m, bcs
+
+    if f_tol == "fifth":  # a tolerance the fifth iteration is the first to meet
+        m, bcs = build()
+        ora = oracle.OracleEnv([m], [], bcs, 1.0e-7)
+        ora.apply_bc_at0()
+        seen = []
+        for n in range(1, 8):
+            m, bcs = build()
+            o = oracle.OracleEnv([m], [], bcs, 1.0e-7)
+            o.apply_bc_at0()
+            o.minimize(1.0e-7, 10.0, max_iter=n, x_tol=1e-30, f_tol=1e-30)
+            free = (bcs[0].bool == 0) & (bcs[1].bool == 0)
+            seen.append(np.abs(o.f[:, free]).max())
+        k = int(np.argmin(seen))
+        f_tol = np.nextafter(seen[k], np.inf)
+    m, bcs = build()
+    env = pb.Env(1, [m], [], bcs, 1.0e-7)
+    ora = oracle.OracleEnv([m], [], bcs, 1.0e-7)
+    ora.apply_bc_at0()
+    pb.apply_bc_at0(env, 0)
+    for _ in range(2):
+        it = pb.minimize(env, pb.QSDrag(1.0e-7, 10.0, max_iter=max_iter, x_tol=1e30, f_tol=f_tol))
+        assert it == ora.minimize(1.0e-7, 10.0, max_iter=max_iter, x_tol=1e30, f_tol=f_tol)
+        _same(env, ora)
+        assert np.array_equal(env.p, ora.p)
+    env.close()
