@@ -1172,20 +1172,22 @@ __global__ void k_gate_final(const GateItem *__restrict__ items, int nitems, int
 }
 
 // peri.jl:587-594 cal_damage: 1 - sum(intact) / intact0
-__global__ void k_damage(int64_t N, const SliceInfo *__restrict__ si,
+// In environment order (map), or in internal order without a map.
+__global__ void k_damage(int64_t n_out, const int64_t *__restrict__ map, const SliceInfo *__restrict__ si,
                          const int32_t *__restrict__ cnt, const uint32_t *__restrict__ words,
                          const int32_t *__restrict__ intact0, const int32_t *__restrict__ tinfo,
                          double *__restrict__ damage) {
-    int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (p >= N) return;
+    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (e >= n_out) return;
+    const int64_t p = map ? map[e] : e;
     if (tinfo[p] < 0) {
-        damage[p] = 0.0;
+        damage[e] = 0.0;
         return;
     }
     int32_t n = cnt[p], c = 0;
     const int64_t wb = si[p >> 5].word + (p & 31);
     for (int32_t w = 0; w * 32 < n; ++w) c += __popc(words[wb + 32 * (int64_t)w]);
-    damage[p] = 1.0 - (double)c / (double)intact0[p];
+    damage[e] = 1.0 - (double)c / (double)intact0[p];
 }
 
 // Fixed partial-reduction width, independent of the device's SM count so
@@ -1442,10 +1444,11 @@ void launch_gate_multi(cudaStream_t st, const GateItem *items, int nitems, int g
     pd::note_launch();
 }
 
-void launch_damage(cudaStream_t st, int64_t N, const SliceInfo *si, const int32_t *cnt,
+void launch_damage(cudaStream_t st, int64_t n_out, const int64_t *map, const SliceInfo *si, const int32_t *cnt,
                    const uint32_t *words, const int32_t *intact0, const int32_t *tinfo,
                    double *damage) {
-    k_damage<<<grid_for(N), kThreads, 0, st>>>(N, si, cnt, words, intact0, tinfo, damage); pd::note_launch();
+    k_damage<<<grid_for(n_out), kThreads, 0, st>>>(n_out, map, si, cnt, words, intact0, tinfo, damage);
+    pd::note_launch();
 }
 
 void launch_sum4(cudaStream_t st, int64_t N, const double4 *a, double *partials, double *out3) {

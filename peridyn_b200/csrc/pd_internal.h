@@ -258,7 +258,8 @@ void launch_gate_multi(cudaStream_t st, const GateItem *items, int nitems, int g
                        const double4 *y, double *partials, int32_t *deformed);
 
 // Damage / diagnostics.
-void launch_damage(cudaStream_t st, int64_t N, const SliceInfo *si, const int32_t *cnt,
+// damage of n_out particles: environment order with map, internal order (map null)
+void launch_damage(cudaStream_t st, int64_t n_out, const int64_t *map, const SliceInfo *si, const int32_t *cnt,
                    const uint32_t *words, const int32_t *intact0, const int32_t *tinfo,
                    double *damage);
 void launch_sum4(cudaStream_t st, int64_t N, const double4 *a, double *partials, double *out3);
