@@ -1673,7 +1673,7 @@ extern "C" pd_status pd_env_get_plastic_strain(pd_env *env, int64_t block, doubl
         for (int32_t k = 0; k < env->cnt_h[p] && r < R; ++k) {
             const int64_t w = wb + 32 * (k / 32);
             if (!((fm[w] >> (k % 32)) & 1u)) continue;
-            edp[(size_t)i * R + r] = e[32 * w + (k % 32)];
+            edp[(size_t)i * R + r] = e[32 * (si[p / 32].word - w0 + k) + (p % 32)];  // slot_index
             ++r;
         }
     }

@@ -127,9 +127,10 @@ struct Geo {
     double *edp_out;
 };
 
-// Per-slot double index of bond slot k of particle p (elasto-plastic edp).
+// Per-slot index of bond slot k of particle p (elasto-plastic edp, partner):
+// the 32 lanes' slots k lie side by side.
 __device__ __forceinline__ int64_t slot_index(const SliceInfo *si, int64_t p, int32_t k) {
-    return ((si[p >> 5].word + 32 * (int64_t)(k >> 5) + (p & 31)) << 5) + (k & 31);
+    return 32 * (si[p >> 5].word + k) + (p & 31);
 }
 
 // Slot of neighbour p in q's family: slots hold descending neighbour
