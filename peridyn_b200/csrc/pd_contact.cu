@@ -115,8 +115,10 @@ __device__ __forceinline__ double jl_fld(double x, double y) {
 // on the GPU it runs on.
 constexpr int kMMBlocks = 148;
 __global__ void __launch_bounds__(kT)
-    k_minmax_partial(int64_t first, int64_t n, const double4 *__restrict__ y, double *__restrict__ part) {
+    k_minmax_partial(int64_t first_a, int64_t n_a, int64_t first_b, int64_t n_b, const double4 *__restrict__ y,
+                     double *__restrict__ part) {
     __shared__ double sh[6][kT];
+    const int64_t first = blockIdx.y ? first_b : first_a, n = blockIdx.y ? n_b : n_a;
     double mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
     for (int64_t i = blockIdx.x * (int64_t)kT + threadIdx.x; i < n; i += (int64_t)kMMBlocks * kT) {
         double4 v = y[first + i];
@@ -141,17 +143,26 @@ __global__ void __launch_bounds__(kT)
         __syncthreads();
     }
     if (threadIdx.x == 0)
-        for (int d = 0; d < 6; ++d) part[6 * blockIdx.x + d] = sh[d][0];
+        for (int d = 0; d < 6; ++d) part[6 * (blockIdx.y * kMMBlocks + blockIdx.x) + d] = sh[d][0];
 }
 
-__global__ void k_minmax_final(const double *__restrict__ part, double *__restrict__ out6) {
-    double r[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
-    for (int b = 0; b < kMMBlocks; ++b)
-        for (int d = 0; d < 3; ++d) {
-            r[d] = fmin(r[d], part[6 * b + d]);
-            r[3 + d] = fmax(r[3 + d], part[6 * b + 3 + d]);
-        }
-    for (int d = 0; d < 6; ++d) out6[d] = r[d];
+// Block b combines the partials of particle range b (exact in any order).
+__global__ void __launch_bounds__(kT) k_minmax_final(const double *__restrict__ part, double *__restrict__ out) {
+    __shared__ double sh[6][kT];
+    static_assert(kMMBlocks <= kT, "one partial per thread");
+    for (int d = 0; d < 6; ++d)
+        sh[d][threadIdx.x] = threadIdx.x < kMMBlocks ? part[6 * (blockIdx.x * kMMBlocks + threadIdx.x) + d]
+                                                     : (d < 3 ? INFINITY : -INFINITY);
+    __syncthreads();
+    for (int s = kT / 2; s > 0; s >>= 1) {
+        if (threadIdx.x < s)
+            for (int d = 0; d < 3; ++d) {
+                sh[d][threadIdx.x] = fmin(sh[d][threadIdx.x], sh[d][threadIdx.x + s]);
+                sh[3 + d][threadIdx.x] = fmax(sh[3 + d][threadIdx.x], sh[3 + d][threadIdx.x + s]);
+            }
+        __syncthreads();
+    }
+    if (threadIdx.x < 6) out[6 * blockIdx.x + threadIdx.x] = sh[threadIdx.x][0];
 }
 
 // ------------------------------- exclusive scan --------------------------
@@ -182,16 +193,38 @@ __global__ void __launch_bounds__(kScanTile)
     if (threadIdx.x == kScanTile - 1) sums[blockIdx.x] = incl;
 }
 
-__global__ void k_scan_sums(int64_t ntiles, int32_t *__restrict__ sums) {
-    // one thread, sequential: tile counts are small
-    if (threadIdx.x != 0) return;
-    int32_t run = 0;
-    for (int64_t t = 0; t < ntiles; ++t) {
-        int32_t s = sums[t];
+// One block: each thread the sum of a run of tiles, the runs scanned.
+__global__ void __launch_bounds__(kScanTile) k_scan_sums(int64_t ntiles, int32_t *__restrict__ sums) {
+    __shared__ int32_t ws[32];
+    const int64_t per = (ntiles + kScanTile - 1) / kScanTile;
+    const int64_t t0 = min(threadIdx.x * per, ntiles), t1 = min(t0 + per, ntiles);
+    int32_t v = 0;
+    for (int64_t t = t0; t < t1; ++t) v += sums[t];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int32_t x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int32_t u = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += u;
+    }
+    if (lane == 31) ws[w] = x;
+    __syncthreads();
+    if (w == 0) {
+        const int32_t s = ws[lane];
+        int32_t y = s;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t u = __shfl_up_sync(0xffffffffu, y, o);
+            if (lane >= o) y += u;
+        }
+        ws[lane] = y - s;
+    }
+    __syncthreads();
+    int32_t run = x + ws[w] - v;
+    for (int64_t t = t0; t < t1; ++t) {
+        const int32_t s = sums[t];
         sums[t] = run;
         run += s;
     }
-    sums[ntiles] = run;
+    if (threadIdx.x == kScanTile - 1) sums[ntiles] = run;
 }
 
 __global__ void k_scan_add(int64_t n, int32_t *__restrict__ out, const int32_t *__restrict__ sums) {
@@ -204,7 +237,7 @@ __global__ void k_scan_add(int64_t n, int32_t *__restrict__ out, const int32_t *
 void scan_exclusive(cudaStream_t st, int64_t n, const int32_t *in, int32_t *out, int32_t *tmp) {
     int64_t nt = std::max<int64_t>(1, (n + kScanTile - 1) / kScanTile);
     k_scan_tiles<<<(unsigned)nt, kScanTile, 0, st>>>(n, in, out, tmp); pd::note_launch();
-    k_scan_sums<<<1, 32, 0, st>>>(nt, tmp); pd::note_launch();
+    k_scan_sums<<<1, kScanTile, 0, st>>>(nt, tmp); pd::note_launch();
     k_scan_add<<<(unsigned)nt, kScanTile, 0, st>>>(n, out, tmp); pd::note_launch();
 }
 
@@ -314,6 +347,86 @@ __global__ void k_c1_select(int64_t n1, int64_t rows, int64_t first2, const int3
     for (int64_t r = 0; r < rows; ++r) nb[r * n1 + i] = r < n ? (int32_t)(first2 + a[r]) : -1;
 }
 
+// The same in one kernel, a warp per set-1 particle, for rows <= kCand / 2:
+// the lanes test the candidate cells' particles (three neighbouring cells of
+// a grid row are one run of clist), the hits are packed into shared memory,
+// and each hit's rank -- how many hits have a larger index -- is its row.  A
+// full buffer is cut to its rows largest before the walk goes on.  Counts
+// the reverse lists on the way.  (A thread per particle, counting, filling
+// and insertion-sorting, left an impact's thousand particles in reach to a
+// few dozen warps: 242 us against 20 for a 17,000-particle sphere.)
+// Set-1 particles in the box (any order: each is worked on by itself).
+__global__ void k_box_list(int64_t first1, int64_t n1, const double4 *__restrict__ y, Box b,
+                           int32_t *__restrict__ list, int32_t *__restrict__ count) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < n1 && in_box(b, y[first1 + i])) list[atomicAdd(count, 1)] = (int32_t)i;
+}
+
+constexpr int kCand = 1024, kSelWarps = 4;
+constexpr int64_t kSelBlocks = 148 * 6;  // 32 KB of buffers a block
+__global__ void __launch_bounds__(32 * kSelWarps)
+    k_c1_select_warp(int64_t first1, int64_t n1, int64_t rows, int64_t first2, const double4 *__restrict__ y, Box b,
+                     double dist2, const int32_t *__restrict__ cstart, const int32_t *__restrict__ clist,
+                     const int32_t *__restrict__ list, const int32_t *__restrict__ count, int32_t *__restrict__ nb,
+                     int32_t *__restrict__ rcnt) {
+    __shared__ int32_t store[kSelWarps][2][kCand];
+    const int lane = threadIdx.x & 31;
+    const int32_t listed = *count;
+    for (int64_t t = (int64_t)blockIdx.x * kSelWarps + (threadIdx.x >> 5); t < listed;
+         t += (int64_t)gridDim.x * kSelWarps) {
+        const int64_t i = list[t];
+        const double4 pi = y[first1 + i];
+        int32_t *buf = store[threadIdx.x >> 5][0], *other = store[threadIdx.x >> 5][1];
+        int32_t n = 0;
+        auto rank_of = [&](int32_t v) {
+            int32_t r = 0;
+            for (int32_t k = 0; k < n; ++k) r += buf[k] > v ? 1 : 0;
+            return r;
+        };
+        const int3 c = box_cell(b, pi);
+        const int x0 = max(c.x - 1, 0), x1 = min(c.x + 1, b.dims.x - 1);
+        for (int z = max(c.z - 1, 0); z <= min(c.z + 1, b.dims.z - 1); ++z)
+            for (int yy = max(c.y - 1, 0); yy <= min(c.y + 1, b.dims.y - 1); ++yy) {
+                const int32_t row = b.dims.x * (yy + b.dims.y * z);
+                const int32_t s1 = cstart[row + x1 + 1];
+                for (int32_t s = cstart[row + x0]; s < s1; s += 32) {
+                    bool hit = false;
+                    int32_t j = 0;
+                    if (s + lane < s1) {
+                        j = clist[s + lane];
+                        const double4 pj = y[first2 + j];
+                        const double a = pi.x - pj.x, bb = pi.y - pj.y, cc = pi.z - pj.z;
+                        hit = a * a + bb * bb + cc * cc < dist2;
+                    }
+                    const uint32_t m = __ballot_sync(0xffffffffu, hit);
+                    if (n + __popc(m) > kCand) {
+                        __syncwarp();
+                        for (int32_t k = lane; k < n; k += 32) {
+                            const int32_t r = rank_of(buf[k]);
+                            if (r < rows) other[r] = buf[k];
+                        }
+                        __syncwarp();
+                        int32_t *t = buf;
+                        buf = other;
+                        other = t;
+                        n = (int32_t)rows;
+                    }
+                    if (hit) buf[n + __popc(m & ((1u << lane) - 1u))] = j;
+                    n += __popc(m);
+                }
+            }
+        __syncwarp();
+        for (int32_t k = lane; k < n; k += 32) {
+            const int32_t j = buf[k], r = rank_of(j);
+            if (r < rows) {
+                nb[r * n1 + i] = (int32_t)(first2 + j);
+                atomicAdd(&rcnt[j], 1);
+            }
+        }
+        __syncwarp();  // the buffers are reused
+    }
+}
+
 // reverse lists: for set-2 particle j, the set-1 particles listing it.
 __global__ void k_rev_count(int64_t n1, int64_t rows, int64_t first2, const int32_t *__restrict__ nb,
                             int32_t *__restrict__ rcnt) {
@@ -326,30 +439,54 @@ __global__ void k_rev_count(int64_t n1, int64_t rows, int64_t first2, const int3
     }
 }
 
+// A warp per listed set-1 particle, its lanes over the rows (which end at the first -1).
 __global__ void k_rev_fill(int64_t n1, int64_t rows, int64_t first1, int64_t first2, const int32_t *__restrict__ nb,
-                           const int32_t *__restrict__ roff, int32_t *__restrict__ cursor, int32_t *__restrict__ rev) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n1) return;
-    for (int64_t r = 0; r < rows; ++r) {
-        int32_t j = nb[r * n1 + i];
-        if (j < 0) break;
-        int32_t s = atomicAdd(&cursor[j - first2], 1);
+                           const int32_t *__restrict__ act, int64_t nact, const int32_t *__restrict__ roff,
+                           int32_t *__restrict__ cursor, int32_t *__restrict__ rev) {
+    const int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    if (t >= nact) return;
+    const int64_t i = act[t];
+    for (int64_t r = threadIdx.x & 31; r < rows; r += 32) {
+        const int32_t j = nb[r * n1 + i];
+        if (j < 0) return;
+        const int32_t s = atomicAdd(&cursor[j - first2], 1);
         rev[roff[j - first2] + s] = (int32_t)(first1 + i);
     }
 }
 
-__global__ void k_rev_sort(int64_t n2, const int32_t *__restrict__ roff, int32_t *__restrict__ rev) {
-    int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j >= n2) return;
-    int32_t o = roff[j], n = roff[j + 1] - o;
+// Each listed reverse list ascending: a warp per list ranks its (distinct) entries
+// in shared memory; lists above the buffer are sorted by one lane.
+__global__ void __launch_bounds__(32 * kSelWarps)
+    k_rev_sort(const int32_t *__restrict__ act, int64_t nact, const int32_t *__restrict__ roff,
+               int32_t *__restrict__ rev) {
+    __shared__ int32_t store[kSelWarps][kCand];
+    const int lane = threadIdx.x & 31;
+    const int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    if (t >= nact) return;
+    const int64_t j = act[t];
+    const int32_t o = roff[j], n = roff[j + 1] - o;
+    if (n < 2) return;
     int32_t *a = rev + o;
-    for (int32_t k = 1; k < n; ++k) {
-        int32_t v = a[k], m = k - 1;
-        while (m >= 0 && a[m] > v) {
-            a[m + 1] = a[m];
-            --m;
+    if (n > kCand) {
+        if (lane) return;
+        for (int32_t k = 1; k < n; ++k) {
+            int32_t v = a[k], m = k - 1;
+            while (m >= 0 && a[m] > v) {
+                a[m + 1] = a[m];
+                --m;
+            }
+            a[m + 1] = v;
         }
-        a[m + 1] = v;
+        return;
+    }
+    int32_t *buf = store[threadIdx.x >> 5];
+    for (int32_t k = lane; k < n; k += 32) buf[k] = a[k];
+    __syncwarp();
+    for (int32_t k = lane; k < n; k += 32) {
+        const int32_t v = buf[k];
+        int32_t r = 0;
+        for (int32_t q = 0; q < n; ++q) r += buf[q] < v ? 1 : 0;
+        a[r] = v;
     }
 }
 
@@ -545,39 +682,17 @@ __global__ void k_c11_force(int64_t first, int64_t n, int64_t nbrows, const int3
     f[p] = fp;
 }
 
-pd_status minmax(pd_env *env, int64_t first, int64_t n, double *out6_host) {
-    if (!env->red.p || env->red.n < 6 * kMMBlocks + 6) PD_TRY(env->red.alloc(6 * kMMBlocks + 6 + 512));
-    k_minmax_partial<<<kMMBlocks, kT, 0, env->st>>>(first, n, env->y.p, env->red.p); pd::note_launch();
-    k_minmax_final<<<1, 1, 0, env->st>>>(env->red.p, env->red.p + 6 * kMMBlocks); pd::note_launch();
+// Bounding boxes (min, max) of one or two particle ranges, with one read-back.
+pd_status minmax(pd_env *env, int ranges, int64_t first_a, int64_t n_a, int64_t first_b, int64_t n_b,
+                 double *out_host) {
+    const int64_t part = 2 * 6 * kMMBlocks;
+    if (!env->red.p || (int64_t)env->red.n < part + 12) PD_TRY(env->red.alloc(part + 12));
+    k_minmax_partial<<<dim3(kMMBlocks, ranges), kT, 0, env->st>>>(first_a, n_a, first_b, n_b, env->y.p, env->red.p);
+    pd::note_launch();
+    k_minmax_final<<<ranges, kT, 0, env->st>>>(env->red.p, env->red.p + part); pd::note_launch();
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(out6_host, env->red.p + 6 * kMMBlocks, 6 * sizeof(double), cudaMemcpyDeviceToHost, env->st));
+    CK(cudaMemcpyAsync(out_host, env->red.p + part, ranges * 6 * sizeof(double), cudaMemcpyDeviceToHost, env->st));
     CK(cudaStreamSynchronize(env->st));
-    return PD_OK;
-}
-
-pd_status build_reverse(pd_env *env, DevContact &dc, int64_t n_src, int64_t src_first, int64_t n_tgt,
-                        int64_t tgt_first, const int32_t *nb, int64_t rows, bool c11) {
-    cudaStream_t st = env->st;
-    CK(cudaMemsetAsync(dc.rev_cnt.p, 0, (n_tgt + 1) * 4, st));
-    if (c11) k_c11_rev_count<<<gridn(n_src), kT, 0, st>>>(src_first, n_src, nb, dc.rev_cnt.p);
-    else k_rev_count<<<gridn(n_src), kT, 0, st>>>(n_src, rows, tgt_first, nb, dc.rev_cnt.p);
-    pd::note_launch();
-    PD_TRY(grow(dc.s_rtmp, (n_tgt + 1 + kScanTile - 1) / kScanTile + 2));
-    scan_exclusive(st, n_tgt + 1, dc.rev_cnt.p, dc.rev_off.p, dc.s_rtmp.p);
-    int32_t total = 0;
-    CK(cudaMemcpyAsync(&total, dc.rev_off.p + n_tgt, 4, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    if (total > dc.rev_cap) {
-        PD_TRY(dc.rev.alloc(total + 1024));
-        dc.rev_cap = total + 1024;
-    }
-    CK(cudaMemsetAsync(dc.rev_cnt.p, 0, (n_tgt + 1) * 4, st));
-    if (c11) k_c11_rev_fill<<<gridn(n_src), kT, 0, st>>>(src_first, n_src, nb, dc.rev_off.p, dc.rev_cnt.p, dc.rev.p);
-    else k_rev_fill<<<gridn(n_src), kT, 0, st>>>(n_src, rows, src_first, tgt_first, nb, dc.rev_off.p, dc.rev_cnt.p,
-                                                 dc.rev.p);
-    pd::note_launch();
-    k_rev_sort<<<gridn(n_tgt), kT, 0, st>>>(n_tgt, dc.rev_off.p, dc.rev.p); pd::note_launch();
-    CK(cudaGetLastError());
     return PD_OK;
 }
 
@@ -591,22 +706,53 @@ __global__ void k_active(int64_t n_src, const int32_t *__restrict__ nb, int64_t 
     if (!self && i < n_tgt && roff[i + 1] > roff[i]) act2[atomicAdd(&counts[1], 1)] = (int32_t)i;
 }
 
-pd_status build_active(pd_env *env, DevContact &dc, bool self) {
+// Reverse lists of the neighbour rows and the lists of particles with
+// contact work.  c11: the one-row reference search of self contact; self:
+// the targets are the sources' own block; counted: rev_cnt already holds the
+// reverse lists' lengths.
+pd_status build_lists(pd_env *env, DevContact &dc, bool c11, bool self, bool counted) {
     cudaStream_t st = env->st;
-    const int64_t n2 = self ? dc.n1 : dc.n2;
-    if ((int64_t)dc.act1.n < dc.n1) PD_TRY(dc.act1.alloc(std::max<int64_t>(dc.n1, 1)));
-    if (!self && (int64_t)dc.act2.n < n2) PD_TRY(dc.act2.alloc(std::max<int64_t>(n2, 1)));
+    const int64_t n_src = dc.n1, n_tgt = self ? dc.n1 : dc.n2;
+    const int64_t src_first = dc.first1, tgt_first = self ? dc.first1 : dc.first2;
+    if (!counted) {
+        CK(cudaMemsetAsync(dc.rev_cnt.p, 0, (n_tgt + 1) * 4, st));
+        if (c11) k_c11_rev_count<<<gridn(n_src), kT, 0, st>>>(src_first, n_src, dc.nb.p, dc.rev_cnt.p);
+        else k_rev_count<<<gridn(n_src), kT, 0, st>>>(n_src, dc.nbrows, tgt_first, dc.nb.p, dc.rev_cnt.p);
+        pd::note_launch();
+    }
+    PD_TRY(grow(dc.s_rtmp, (n_tgt + 1 + kScanTile - 1) / kScanTile + 2));
+    scan_exclusive(st, n_tgt + 1, dc.rev_cnt.p, dc.rev_off.p, dc.s_rtmp.p);
+    if ((int64_t)dc.act1.n < n_src) PD_TRY(dc.act1.alloc(std::max<int64_t>(n_src, 1)));
+    if (!self && (int64_t)dc.act2.n < n_tgt) PD_TRY(dc.act2.alloc(std::max<int64_t>(n_tgt, 1)));
     if (!dc.act_n.p) PD_TRY(dc.act_n.alloc(2));
     CK(cudaMemsetAsync(dc.act_n.p, 0, 2 * sizeof(int32_t), st));
-    const int64_t n = std::max(dc.n1, n2);
-    k_active<<<gridn(n), kT, 0, st>>>(dc.n1, dc.nb.p, n2, dc.rev_off.p, self ? 1 : 0, dc.act1.p,
+    const int64_t n = std::max(n_src, n_tgt);
+    k_active<<<gridn(n), kT, 0, st>>>(n_src, dc.nb.p, n_tgt, dc.rev_off.p, self ? 1 : 0, dc.act1.p,
                                       self ? nullptr : dc.act2.p, dc.act_n.p);
     pd::note_launch();
-    int32_t h[2] = {0, 0};
+    int32_t total = 0, h[2] = {0, 0};
+    CK(cudaMemcpyAsync(&total, dc.rev_off.p + n_tgt, 4, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(h, dc.act_n.p, sizeof(h), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemsetAsync(dc.rev_cnt.p, 0, (n_tgt + 1) * 4, st));  // the fill's cursors
     CK(cudaStreamSynchronize(st));
     dc.nact1 = h[0];
     dc.nact2 = self ? 0 : h[1];
+    if (total > dc.rev_cap) {
+        PD_TRY(dc.rev.alloc(total + 1024));
+        dc.rev_cap = total + 1024;
+    }
+    if (total == 0) return PD_OK;
+    if (c11)
+        k_c11_rev_fill<<<gridn(n_src), kT, 0, st>>>(src_first, n_src, dc.nb.p, dc.rev_off.p, dc.rev_cnt.p, dc.rev.p);
+    else
+        k_rev_fill<<<gridn(32 * dc.nact1), kT, 0, st>>>(n_src, dc.nbrows, src_first, tgt_first, dc.nb.p, dc.act1.p,
+                                                        dc.nact1, dc.rev_off.p, dc.rev_cnt.p, dc.rev.p);
+    pd::note_launch();
+    const int64_t nt = self ? dc.nact1 : dc.nact2;  // the targets with reverse entries are among these
+    k_rev_sort<<<gridn(32 * nt, 32 * kSelWarps), 32 * kSelWarps, 0, st>>>(self ? dc.act1.p : dc.act2.p, nt,
+                                                                         dc.rev_off.p, dc.rev.p);
+    pd::note_launch();
+    CK(cudaGetLastError());
     return PD_OK;
 }
 
@@ -614,9 +760,8 @@ pd_status update12(pd_env *env, const HostContact &hc, DevContact &dc) {
     cudaStream_t st = env->st;
     const int64_t n1 = dc.n1, n2 = dc.n2;
     CK(cudaMemsetAsync(dc.nb.p, 0xff, (size_t)n1 * dc.rows * 4, st));
-    double m1[6], m2[6];
-    PD_TRY(minmax(env, dc.first1, n1, m1));
-    PD_TRY(minmax(env, dc.first2, n2, m2));
+    double mm[12], *m1 = mm, *m2 = mm + 6;
+    PD_TRY(minmax(env, 2, dc.first1, n1, dc.first2, n2, mm));
     // contacts.jl:403-416 collision_box
     const double skin = hc.distance;
     Box b;
@@ -626,10 +771,7 @@ pd_status update12(pd_env *env, const HostContact &hc, DevContact &dc) {
     }
     double bvol = (b.hi[0] - b.lo[0]) * (b.hi[1] - b.lo[1]) * (b.hi[2] - b.lo[2]);
     dc.has_neighs = true;
-    if (bvol < 0.0) {
-        PD_TRY(build_reverse(env, dc, n1, dc.first1, n2, dc.first2, dc.nb.p, dc.rows, false));
-        return build_active(env, dc, false);
-    }
+    if (bvol < 0.0) return build_lists(env, dc, false, false, false);
     double cell = hc.distance * (1.0 + 1e-9);
     int dims[3];
     double tot = 1.0;
@@ -663,6 +805,20 @@ pd_status update12(pd_env *env, const HostContact &hc, DevContact &dc) {
     scan_exclusive(st, ncell + 1, ccount.p, cstart.p, tmp.p);
     k_c2_scatter<<<gridn(n2), kT, 0, st>>>(n2, cell_of.p, cstart.p, cursor.p, clist.p); pd::note_launch();
     const double dist2 = hc.distance * hc.distance;
+    if (dc.rows <= kCand / 2) {
+        CK(cudaMemsetAsync(dc.rev_cnt.p, 0, (n2 + 1) * 4, st));
+        PD_TRY(grow(c1cnt, n1 + 1));  // the listed particles, then their number
+        CK(cudaMemsetAsync(c1cnt.p + n1, 0, 4, st));
+        k_box_list<<<gridn(n1), kT, 0, st>>>(dc.first1, n1, env->y.p, b, c1cnt.p, c1cnt.p + n1); pd::note_launch();
+        const int64_t blocks = std::min<int64_t>(kSelBlocks, (n1 + kSelWarps - 1) / kSelWarps);
+        k_c1_select_warp<<<(unsigned)blocks, 32 * kSelWarps, 0, st>>>(
+            dc.first1, n1, dc.rows, dc.first2, env->y.p, b, dist2, cstart.p, clist.p, c1cnt.p, c1cnt.p + n1, dc.nb.p,
+            dc.rev_cnt.p);
+        pd::note_launch();
+        CK(cudaGetLastError());
+        return build_lists(env, dc, false, false, true);
+    }
+    // more rows than the selection's buffer holds: count, fill, sort
     PD_TRY(grow(c1cnt, n1 + 1));
     PD_TRY(grow(c1off, n1 + 1));
     CK(cudaMemsetAsync(c1cnt.p, 0, (n1 + 1) * 4, st));
@@ -677,14 +833,13 @@ pd_status update12(pd_env *env, const HostContact &hc, DevContact &dc) {
                                                     nullptr, c1off.p, cand.p); pd::note_launch();
     k_c1_select<<<gridn(n1), kT, 0, st>>>(n1, dc.rows, dc.first2, c1off.p, cand.p, dc.nb.p); pd::note_launch();
     CK(cudaGetLastError());
-    PD_TRY(build_reverse(env, dc, n1, dc.first1, n2, dc.first2, dc.nb.p, dc.rows, false));
-    return build_active(env, dc, false);
+    return build_lists(env, dc, false, false, false);
 }
 
 pd_status update11(pd_env *env, const HostContact &hc, DevContact &dc, int64_t max_part) {
     cudaStream_t st = env->st;
     double m[6];
-    PD_TRY(minmax(env, dc.first1, dc.n1, m));
+    PD_TRY(minmax(env, 1, dc.first1, dc.n1, 0, 0, m));
     RefCells rc;
     for (int d = 0; d < 3; ++d) rc.mn[d] = m[d];
     rc.h = hc.distance;
@@ -702,9 +857,7 @@ pd_status update11(pd_env *env, const HostContact &hc, DevContact &dc, int64_t m
     }
     CK(cudaGetLastError());
     dc.has_neighs = true;
-    PD_TRY(build_reverse(env, dc, dc.n1, dc.first1, dc.n1, dc.first1, dc.nb.p, dc.nbrows,
-                         hc.kind != PD_CONTACT_11_ORDERED));
-    return build_active(env, dc, true);
+    return build_lists(env, dc, hc.kind != PD_CONTACT_11_ORDERED, true, false);
 }
 
 }  // namespace
