@@ -881,6 +881,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 1)
         const uint64_t nz = 0x8000000000000000ull;
         const bool neg = (uint64_t)__double_as_longlong(f0.x) == nz || (uint64_t)__double_as_longlong(f0.y) == nz ||
                          (uint64_t)__double_as_longlong(f0.z) == nz;
+        __syncthreads();  // every warp has read f before one writes it
         if (__any_sync(0xffffffffu, neg)) {  // the same lanes in every warp
             if (w == 0 && ti >= 0) force_particle_general(g, p, ti, kind, y, mth, win, wout, f);
             return;
