@@ -15,6 +15,7 @@
 
 #include "pd_ieee.h"
 #include "pd_internal.h"
+#include "pd_launch.h"
 
 namespace pd {
 
@@ -327,17 +328,18 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 3 : 1)
     k_theta_slice(Geo g, const double4 *__restrict__ y, const uint32_t *__restrict__ win, double2 *__restrict__ mth,
                   int64_t s0) {
     __shared__ double term[kThetaTile][32];
-    if (g.stop && *g.stop) return;
     const int64_t s = s0 + blockIdx.x;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t p = 32 * s + lane;
     const int32_t ti = g.tinfo[p];
     const int32_t tb = __reduce_max_sync(0xffffffffu, ti);
     const int kind = tb >= 0 ? g.blocks[tb >> 8].kind : PD_MAT_SKIP;
-    if (kind != PD_MAT_ORDINARY_STATE_BASED && kind != PD_MAT_ELASTO_PLASTIC) return;
-    const double4 xp = ld4(g.x4 + p), yp = ld4(y + p);
-    const double c_i = ti >= 0 ? 3.0 / mth[p].x : 0.0;
     const int32_t n = g.cnt[p];
+    const double4 xp = ld4(g.x4 + p);
+    pdl_enter();  // before any return: the next kernel may wait for this one only
+    if ((kind != PD_MAT_ORDINARY_STATE_BASED && kind != PD_MAT_ELASTO_PLASTIC) || (g.stop && *g.stop)) return;
+    const double4 yp = ld4(y + p);
+    const double c_i = ti >= 0 ? 3.0 / mth[p].x : 0.0;
     const int32_t L = (int32_t)__reduce_max_sync(0xffffffffu, (unsigned)n);
     const SliceInfo d = g.si[s];
     const bool st = d.mode == kStencil;
@@ -855,7 +857,6 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 1)
                   const uint32_t *__restrict__ win, uint32_t *__restrict__ wout, double4 *__restrict__ f,
                   int accumulate, int32_t cap, int64_t s0) {
     extern __shared__ double term[];  // [slot][component][lane], then the broken bits [word][lane]
-    if (g.stop && *g.stop) return;
     const int64_t s = s0 + blockIdx.x;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t p = 32 * s + lane;
@@ -865,7 +866,8 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 1)
     // every particle of a slice belongs to one block (padding: -1)
     const int32_t tb = __reduce_max_sync(0xffffffffu, ti);
     const int kind = tb >= 0 ? g.blocks[tb >> 8].kind : PD_MAT_SKIP;
-    if (kind == PD_MAT_ELASTO_PLASTIC || L > cap) return;
+    pdl_enter();  // before any return: the next kernel may wait for this one only
+    if (kind == PD_MAT_ELASTO_PLASTIC || L > cap || (g.stop && *g.stop)) return;
     const int32_t words = (L + 31) >> 5;
     uint32_t *brk = reinterpret_cast<uint32_t *>(term + 96 * (int64_t)cap);
     const uint32_t *wi = win + d.word + lane;
@@ -1044,6 +1046,7 @@ __global__ void __launch_bounds__(256)
               double4 *__restrict__ y, const double *__restrict__ mass, double4 *__restrict__ p,
               const __grid_constant__ FusedBCs b, int64_t ts) {
     const int64_t i = blockIdx.x * (int64_t)256 + threadIdx.x;
+    pdl_enter();
     if (i >= N) return;
     const double4 fi = f[i];
     double4 vi = v[i], yi = y[i];
@@ -1342,8 +1345,8 @@ void launch_theta_serial(cudaStream_t st, const Geo &g, const double4 *y, const 
                          double2 *mth, int64_t p0, int64_t p1) {
     if (p1 <= p0) return;
     const int64_t S = (p1 - p0) / 32;
-    if (wide_slices(S)) k_theta_slice<16><<<(unsigned)S, 512, 0, st>>>(g, y, win, mth, p0 / 32);
-    else k_theta_slice<8><<<(unsigned)S, 256, 0, st>>>(g, y, win, mth, p0 / 32);
+    if (wide_slices(S)) launch_dep(k_theta_slice<16>, (unsigned)S, 512, st, g, y, win, mth, p0 / 32);
+    else launch_dep(k_theta_slice<8>, (unsigned)S, 256, st, g, y, win, mth, p0 / 32);
     pd::note_launch();
 }
 
@@ -1376,9 +1379,9 @@ void launch_force_serial(cudaStream_t st, const Geo &g, const double4 *y, const 
     const int64_t S = (p1 - p0) / 32;
     force_slice_attrs();
     if (wide_slices(S))
-        k_force_slice<16><<<(unsigned)S, 512, sm, st>>>(g, y, mth, win, wout, f, accumulate, cap, p0 / 32);
+        launch_dep_smem(k_force_slice<16>, (unsigned)S, 512, sm, st, g, y, mth, win, wout, f, accumulate, cap, p0 / 32);
     else
-        k_force_slice<8><<<(unsigned)S, 256, sm, st>>>(g, y, mth, win, wout, f, accumulate, cap, p0 / 32);
+        launch_dep_smem(k_force_slice<8>, (unsigned)S, 256, sm, st, g, y, mth, win, wout, f, accumulate, cap, p0 / 32);
     pd::note_launch();
     if (g.has_ep || g.max_slots > cap) {
         k_force_serial<<<grid_for(p1 - p0), kThreads, 0, st>>>(g, y, mth, win, wout, f, accumulate, cap, p0, p1);
@@ -1389,9 +1392,8 @@ void launch_force_serial(cudaStream_t st, const Geo &g, const double4 *y, const 
 void launch_advance(cudaStream_t st, int64_t N, double c, double dt, bool post, bool pre, const double4 *f,
                     double4 *v, double4 *y, const double *mass, double4 *p, const FusedBCs &bcs, int64_t ts) {
     const unsigned g = grid_for(N, 256);
-    if (post && pre) k_advance<true, true><<<g, 256, 0, st>>>(N, c, dt, f, v, y, mass, p, bcs, ts);
-    else if (post) k_advance<true, false><<<g, 256, 0, st>>>(N, c, dt, f, v, y, mass, p, bcs, ts);
-    else k_advance<false, true><<<g, 256, 0, st>>>(N, c, dt, f, v, y, mass, p, bcs, ts);
+    auto kern = post && pre ? k_advance<true, true> : post ? k_advance<true, false> : k_advance<false, true>;
+    launch_dep(kern, g, 256, st, N, c, dt, f, v, y, mass, p, bcs, ts);
     pd::note_launch();
 }
 

@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "pd_env_impl.h"
+#include "pd_launch.h"
 
 using namespace pd;
 
@@ -140,6 +141,7 @@ __global__ void __launch_bounds__(256)
                double ss, double a, double f_tol, double x_tol, double *__restrict__ partial, QsState *qs) {
     __shared__ double sf[256], sy[256];
     __shared__ bool last;
+    pdl_enter();
     if (*(volatile int32_t *)&qs->done) return;
     double mf = 0.0, my = 0.0;
     for (int64_t i = blockIdx.x * 256 + threadIdx.x; i < N; i += (int64_t)kRedBlocks * 256) {
@@ -448,8 +450,10 @@ extern "C" pd_status pd_env_qsdrag(pd_env *env, double step_size, double drag, i
         const int cur0 = env->cur, ecur0 = env->ecur;
         for (int64_t i = 0; i < m; ++i) {
             PD_TRY(update_acc_serial(env, false, &qs->done));
-            k_qs_apply<<<kRedBlocks, 256, 0, st>>>(N, env->free_mask.p, env->f.p, env->opt.p, env->y.p, lambda, kk,
-                                                   step_size, a, f_tol, x_tol, env->red.p, qs); pd::note_launch();
+            launch_dep(k_qs_apply, kRedBlocks, 256, st, (int64_t)N, (const int32_t *)env->free_mask.p,
+                       (const double4 *)env->f.p, env->opt.p, env->y.p, lambda, kk, step_size, a, f_tol, x_tol,
+                       env->red.p, qs);
+            pd::note_launch();
         }
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(&h, qs, sizeof(h), cudaMemcpyDeviceToHost, st));
