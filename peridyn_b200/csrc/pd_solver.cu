@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(256)
     k_qs_apply(int64_t N, const int32_t *__restrict__ freem, const double4 *__restrict__ f,
                double4 *__restrict__ opt, double4 *__restrict__ y, double lambda, double kk,
                double ss, double a, double f_tol, double x_tol, double *__restrict__ partial, QsState *qs) {
-    __shared__ double sf[256], sy[256];
+    __shared__ double sf[8], sy[8];
     __shared__ bool last;
     pdl_enter();
     if (*(volatile int32_t *)&qs->done) return;
@@ -160,17 +160,32 @@ __global__ void __launch_bounds__(256)
         opt[i] = make_double4(o[0], o[1], o[2], 0.0);
         y[i] = make_double4(yy[0], yy[1], yy[2], yi.w);
     }
+    // the block's maxima in sf[0], sy[0]: within the warps, then over them
     auto reduce = [&](double vf, double vy) {
-        sf[threadIdx.x] = vf;
-        sy[threadIdx.x] = vy;
-        __syncthreads();
-        for (int s = 128; s > 0; s >>= 1) {
-            if (threadIdx.x < s) {
-                sf[threadIdx.x] = nanmax(sf[threadIdx.x], sf[threadIdx.x + s]);
-                sy[threadIdx.x] = nanmax(sy[threadIdx.x], sy[threadIdx.x + s]);
-            }
-            __syncthreads();
+        for (int o = 16; o; o >>= 1) {
+            vf = nanmax(vf, __shfl_xor_sync(0xffffffffu, vf, o));
+            vy = nanmax(vy, __shfl_xor_sync(0xffffffffu, vy, o));
         }
+        const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        if (lane == 0) {
+            sf[wid] = vf;
+            sy[wid] = vy;
+        }
+        __syncthreads();
+        if (wid == 0) {
+            vf = lane < 8 ? sf[lane] : 0.0;
+            vy = lane < 8 ? sy[lane] : 0.0;
+            for (int o = 4; o; o >>= 1) {
+                vf = nanmax(vf, __shfl_xor_sync(0xffffffffu, vf, o));
+                vy = nanmax(vy, __shfl_xor_sync(0xffffffffu, vy, o));
+            }
+            __syncwarp();
+            if (lane == 0) {
+                sf[0] = vf;
+                sy[0] = vy;
+            }
+        }
+        __syncthreads();
     };
     reduce(mf, my);
     if (threadIdx.x == 0) {
