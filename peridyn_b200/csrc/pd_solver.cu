@@ -457,7 +457,7 @@ extern "C" pd_status pd_env_qsdrag(pd_env *env, double step_size, double drag, i
     const bool ep = env->geo().has_ep != 0;
     for (int64_t batch = 2; h.iters < max_iter && !h.done; batch = std::min(2 * batch, kQsBatch)) {
         PD_TRY(refresh_deformed(env));
-        bool known = env->hc.empty();
+        bool known = env->hc.empty() && !env->prof;  // (profiling counts the iterations that run)
         for (size_t b = 0; b < env->hb.size() && !env->gate_hold; ++b)
             if (env->hb[b].kind != PD_MAT_SKIP && !env->deformed_h[b]) known = false;
         const int64_t m = known ? std::min(batch, max_iter - h.iters) : 1;
