@@ -343,7 +343,8 @@ PD_API pd_status pd_env_profile_read(pd_env *env, double *total_ms, int64_t *lau
 /* Kernel shape of the throughput modes (extension): warps per 32-particle
  * slice (1, 2, 4, 8) and bonds in flight per thread (FP32C: 2 or 4, FP64:
  * 1 or 2).  (0, 0) returns to the autotuner, which times every shape on
- * the first step and caches the fastest per problem size. */
+ * the first step -- for up to 65,536 particles also 16 warps per slice --
+ * and caches the fastest per problem size. */
 PD_API pd_status pd_env_set_kernel_shape(pd_env *env, int32_t warps_per_slice, int32_t unroll);
 /* The shape the throughput path runs with (after autotuning); (0, 0)
  * before the first throughput-mode step or in the serial mode. */
