@@ -16,6 +16,7 @@
 #include "pd_ieee.h"
 #include "pd_internal.h"
 #include "pd_launch.h"
+#include "pd_slots.h"
 
 namespace pd {
 
@@ -771,7 +772,7 @@ __device__ __forceinline__ void evaluate_slice(const Geo &g, const DevBlock &B, 
         bool fast = sqrt_rcp_rn(X1 * X1 + X2 * X2 + X3 * X3, xij, rx) && own_ok;
         fast = sqrt_rcp_rn(Y1 * Y1 + Y2 * Y2 + Y3 * Y3, yij, ry) && fast;
         fast = (uint32_t)hi_word(r.x.w) < ((1023u + 100u) << 20) && fast;
-        const PairParam pp = MULTI ? g.pairs[B.pair_base + tp + (g.tinfo[r.q] & 255) * B.nt] : pp0;
+        const PairParam pp = MULTI ? g.pairs[slot_pair(B.pair_base, B.nt, tp, g.tinfo[r.q], live)] : pp0;
         const double ext = yij - xij;
         const double s = div_rn(ext, xij, rx);
         within = s < pp.cs;

@@ -1,0 +1,54 @@
+"""The serial mode's slice kernels in environments of several blocks, some
+with several types, whose particle counts leave padding lanes and whose
+stencils reach into the neighbouring block's records: bit-identical to the
+oracle's serial loop."""
+import numpy as np
+import pytest
+
+import peridyn_b200 as pb
+from peridyn_b200 import lattice
+
+pytestmark = pytest.mark.gpu
+
+
+def block(law, dims, ntypes, first_type, offset, factor=2.3, seed=5):
+    h = 1.0e-3
+    x, vol = lattice.cuboid(*dims, h, jitter=2.0e-5, seed=seed)
+    x = np.asfortranarray(x + np.array([[offset], [0.0], [0.0]]))
+    v = lattice.gaussian_pulse(x, 40.0, 2.0e-3)
+    t = (first_type + (np.arange(x.shape[1]) * 7 // 5) % ntypes).astype(np.int64)
+    gen = pb.GeneralMaterial(x.copy(order="F"), v, x, vol, t, factor * h, max_neigh=200)
+    pairs = ntypes * (ntypes + 1) // 2
+    r = np.linspace(1.0, 1.2, pairs)
+    rho = list(np.linspace(2000.0, 2600.0, ntypes))
+    cs = list(0.003 * r)
+    if law == "pmb":
+        return pb.PeridynamicsMaterial(gen, pb.BondBasedSpecific(list(14.9e9 * r), cs, rho))
+    return pb.PeridynamicsMaterial(gen, pb.OrdinaryStateBasedSpecific(list(20e9 * r), list(9e9 * r), cs, rho))
+
+
+def three_blocks(law, sizes):
+    other = "lps" if law == "pmb" else "pmb"
+    return [block(other, sizes[0], 3, 1, 0.0), block(law, sizes[1], 2, 4, 0.03, seed=6),
+            block(law, sizes[2], 5, 6, 0.06, seed=7)]
+
+
+@pytest.mark.parametrize("law", ["pmb", "lps"])
+@pytest.mark.parametrize("sizes", [((7, 3, 3), (5, 5, 5), (3, 3, 3)), ((8, 4, 4), (9, 7, 5), (4, 4, 2)),
+                                   ((3, 1, 1), (26, 16, 15), (1, 2, 3))])
+def test_blocks_of_several_types(oracle, law, sizes):
+    mats = three_blocks(law, sizes)
+    env = pb.Env(1, mats, [], [], 2.0e-8)
+    ora = oracle.OracleEnv(mats, [], [], 2.0e-8)
+    pb.update_acc(env)
+    ora.update_acc()
+    pb.velocity_verlet_step(env, nsteps=15)
+    for _ in range(15):
+        ora.vv_step()
+    y, v, f, _ = env.get_state()
+    assert np.array_equal(f, ora.f)
+    assert np.array_equal(v, ora.v)
+    assert np.array_equal(y, ora.y)
+    for b, B in enumerate(ora.blocks):
+        assert np.array_equal(env._family(b)[1], B.intact.astype(bool))
+    env.close()
