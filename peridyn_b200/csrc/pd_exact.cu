@@ -336,20 +336,18 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 3 : 1)
     const int32_t tb = __reduce_max_sync(0xffffffffu, ti);
     const int kind = tb >= 0 ? g.blocks[tb >> 8].kind : PD_MAT_SKIP;
     const int32_t n = g.cnt[p];
-    const double4 xp = ld4(g.x4 + p);
+    const int32_t own = lane_record((int32_t)p, ti);
+    const double4 xp = ld4(g.x4 + own);
     pdl_enter();  // before any return: the next kernel may wait for this one only
     if ((kind != PD_MAT_ORDINARY_STATE_BASED && kind != PD_MAT_ELASTO_PLASTIC) || (g.stop && *g.stop)) return;
-    const double4 yp = ld4(y + p);
+    const double4 yp = ld4(y + own);
     const double c_i = ti >= 0 ? 3.0 / mth[p].x : 0.0;
     const int32_t L = (int32_t)__reduce_max_sync(0xffffffffu, (unsigned)n);
     const SliceInfo d = g.si[s];
     const bool st = d.mode == kStencil;
     const int32_t *nb = g.nbr + d.nbr + (st ? 0 : lane);
     const uint32_t *wi = win + d.word + lane;
-    auto neighbour = [&](int32_t k) -> int32_t {
-        if (k >= n) return (int32_t)p;
-        return st ? (int32_t)p + __ldg(nb + k) : __ldg(nb + 32 * k);
-    };
+    auto entry = [&](int32_t k) { return __ldg(nb + (st ? k : 32 * k)); };  // (a slice stores all its slots)
     auto evaluate = [&](const double4 &xq, const double4 &yq, double &t) -> bool {
         const double X1 = xq.x - xp.x, X2 = xq.y - xp.y, X3 = xq.z - xp.z;
         const double Y1 = yq.x - yp.x, Y2 = yq.y - yp.y, Y3 = yq.z - yp.z;
@@ -366,9 +364,10 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 3 : 1)
         if (base) __syncthreads();
         for (int32_t j = j0; j < j1; j += 2) {
             const int32_t ka = base + j, kb = base + min(j + 1, j1 - 1);
-            const int32_t qa = neighbour(ka), qb = neighbour(kb);
+            const int32_t na = entry(ka), nb2 = entry(kb);
             const bool la = ka < n && ((wi[32 * (ka >> 5)] >> (ka & 31)) & 1u);
             const bool lb = kb < n && ((wi[32 * (kb >> 5)] >> (kb & 31)) & 1u);
+            const int32_t qa = slot_record(st, own, na, la), qb = slot_record(st, own, nb2, lb);
             const double4 xa = ld4(g.x4 + qa), ya = ld4(y + qa), xb = ld4(g.x4 + qb), yb = ld4(y + qb);
             double ta, tb2;
             const bool ea = evaluate(xa, ya, ta), eb = evaluate(xb, yb, tb2);
@@ -734,8 +733,9 @@ __device__ __forceinline__ void evaluate_slice(const Geo &g, const DevBlock &B, 
                                                const uint32_t *__restrict__ win, double *term, uint32_t *brk) {
     constexpr bool PMB = KIND == PD_MAT_BOND_BASED;
     const int tp = ti >= 0 ? ti & 255 : 0;
-    const double4 xp = ld4(g.x4 + p), yp = ld4(y + p);
-    const double2 mp = PMB ? make_double2(0.0, 0.0) : mth[p];
+    const int32_t own = lane_record((int32_t)p, ti);
+    const double4 xp = ld4(g.x4 + own), yp = ld4(y + own);
+    const double2 mp = PMB ? make_double2(0.0, 0.0) : mth[own];
     const double rho_p = g.tdens[B.type_base + tp];
     const PairParam pp0 = g.pairs[B.pair_base + tp + tp * B.nt];
     const double c11 = B.c11;
@@ -746,12 +746,7 @@ __device__ __forceinline__ void evaluate_slice(const Geo &g, const DevBlock &B, 
     // warp w evaluates the contiguous slots [k0, k1)
     const int32_t per = (L + NW - 1) / NW, k0 = min(w * per, L), k1 = min(k0 + per, L);
     if (k0 >= k1) return;
-    // (a stencil offset is in range for every lane with bonds)
-    const int32_t some = n > 0 ? -1 : 0;
-    auto neighbour = [&](int32_t k) -> int32_t {
-        if (ST) return (int32_t)p + (__ldg(nb + k) & some);
-        return k < n ? __ldg(nb + 32 * k) : (int32_t)p;
-    };
+    auto entry = [&](int32_t k) { return __ldg(nb + (ST ? k : 32 * k)); };  // (a slice stores all its slots)
     auto load = [&](int32_t q) {
         SlotIn r;
         r.x = ld4(g.x4 + q);
@@ -814,19 +809,19 @@ __device__ __forceinline__ void evaluate_slice(const Geo &g, const DevBlock &B, 
     };
     // two slots at a time, their chains side by side (a chain is some 35
     // dependent FP64 operations of 16 cycles, and 16 warps fit an SM)
-    int32_t qa = neighbour(k0), qb = neighbour(min(k0 + 1, k1 - 1));
+    int32_t na = entry(k0), nb2 = entry(min(k0 + 1, k1 - 1));
     for (int32_t k = k0; k < k1;) {
         const int32_t word = k >> 5, kw = min(k1, (word + 1) << 5);  // slots of one intact word
         bits = 32 * word < n ? wi[32 * word] : 0u;
         gone = 0;
         for (; k < kw; k += 2) {
             const bool two = k + 1 < kw;
-            const SlotIn ra = load(qa), rb = load(two ? qb : qa);
-            const int32_t next = two ? k + 2 : k + 1;
-            qa = neighbour(min(next, k1 - 1));
-            qb = neighbour(min(next + 1, k1 - 1));
             const uint32_t b2 = bits >> (k & 31);
-            const bool la = (b2 & 1u) != 0u, lb = (b2 & 2u) != 0u;
+            const bool la = (b2 & 1u) != 0u, lb = two && (b2 & 2u) != 0u;
+            const SlotIn ra = load(slot_record(ST, own, na, la)), rb = load(slot_record(ST, own, nb2, lb));
+            const int32_t next = two ? k + 2 : k + 1;
+            na = entry(min(next, k1 - 1));
+            nb2 = entry(min(next + 1, k1 - 1));
             double a0, a1, a2, b0, b1, bz;
             bool wa, wb;
             const bool ea = evaluate(ra, la, a0, a1, a2, wa), eb = evaluate(rb, lb, b0, b1, bz, wb);
@@ -880,7 +875,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 1)
         return;
     }
     if (accumulate) {
-        const double4 f0 = f[p];
+        const double4 f0 = f[lane_record((int32_t)p, ti)];
         const uint64_t nz = 0x8000000000000000ull;
         const bool neg = (uint64_t)__double_as_longlong(f0.x) == nz || (uint64_t)__double_as_longlong(f0.y) == nz ||
                          (uint64_t)__double_as_longlong(f0.z) == nz;
@@ -920,7 +915,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 1)
     const int32_t kmax = (int32_t)__reduce_max_sync(0xffffffffu, (unsigned)kp);
     const double *T = term + 32 * w + lane;
     double *fo = reinterpret_cast<double *>(f + p);
-    double a = accumulate ? fo[w] : 0.0;
+    double a = accumulate && ti >= 0 ? fo[w] : 0.0;
 #pragma unroll 8
     for (int32_t k = L - 1; k >= kmin; --k) {
         const double t = T[96 * k];

@@ -2,8 +2,9 @@
 // (peridyn_b200/csrc/pd_slots.h): two adjacent multi-type lattice blocks,
 // particle counts on and off the multiples of 32, stencil slices built as
 // the library builds them (the union of the lanes' offsets).  Every slot of
-// every lane, used or not, must index inside the block's pair table, and a
-// used slot must find its own pair.  Prints "ok <slots>" or the first
+// every lane, used or not, must read a particle's record of its own block
+// and index inside the block's pair table, and a used slot must find its own
+// neighbour and pair.  Prints "ok <slots>" or the first
 // failure; exit status 0 on success.
 #include <algorithm>
 #include <cstdio>
@@ -70,7 +71,14 @@ void check(std::vector<Block> blocks, double r) {
                 for (const int o : offs) {
                     const int p = s + l;
                     const bool live = std::binary_search(fam[l].begin(), fam[l].end(), p + o, std::greater<int>());
-                    const int q = fam[l].empty() ? p : p + o;
+                    const int q = slot_record(true, lane_record(p, tinfo[p]), o, live);
+                    const int qe = slot_record(false, lane_record(p, tinfo[p]), live ? p + o : 0, live);
+                    if (q < b.first || q >= b.first + b.n || q != qe || (live && q != p + o)) {
+                        if (!failures++)
+                            std::printf("lane %d of slice %d, offset %d: record %d (explicit %d) outside [%d, %d)\n", l,
+                                        s / 32, o, q, qe, b.first, b.first + b.n);
+                        continue;
+                    }
                     const int tp = tinfo[p] >= 0 ? tinfo[p] & 255 : 0;
                     const int k = slot_pair(b.pair_base, b.nt, tp, tinfo[q], live);
                     ++checked;

@@ -52,3 +52,36 @@ def test_blocks_of_several_types(oracle, law, sizes):
     for b, B in enumerate(ora.blocks):
         assert np.array_equal(env._family(b)[1], B.intact.astype(bool))
     env.close()
+
+
+@pytest.mark.parametrize("entry", ["pd_force_density_device_static", "pd_force_density_device"])
+@pytest.mark.parametrize("law", ["pmb", "lps"])
+def test_one_block_of_several_through_device_pointers(oracle, law, entry):
+    """Each block by itself, in turn; the other blocks' positions are NaN."""
+    import ctypes
+
+    import torch
+
+    from peridyn_b200 import _abi
+
+    mats = three_blocks(law, ((7, 3, 3), (9, 7, 5), (3, 3, 3)))
+    env = pb.Env(1, mats, [], [], 2.0e-8)
+    ora = oracle.OracleEnv(mats, [], [], 2.0e-8)
+    rng = np.random.default_rng(4)
+    ora.y[:] = ora.y + rng.normal(0.0, 1e-6, size=ora.y.shape)
+    f0 = np.asfortranarray(rng.normal(0.0, 1.0, size=ora.y.shape))
+    ora.f[:] = f0
+    for b, B in enumerate(ora.blocks):
+        own = slice(B.off, B.off + B.n)
+        y = np.full_like(ora.y, np.nan)
+        y[:, own] = ora.y[:, own]
+        yd = torch.from_numpy(np.ascontiguousarray(y.T)).cuda()
+        fd = torch.from_numpy(np.ascontiguousarray(f0.T)).cuda()
+        _abi.check(getattr(_abi.lib(), entry)(env._h, b, ctypes.c_void_p(fd.data_ptr()),
+                                              ctypes.c_void_p(yd.data_ptr()), None))
+        f = fd.cpu().numpy().T
+        ora.force_density_T(B)
+        assert np.array_equal(f[:, own], ora.f[:, own])
+        assert np.array_equal(np.delete(f, np.r_[own], axis=1), np.delete(f0, np.r_[own], axis=1))
+        assert np.array_equal(env._family(b)[1], B.intact.astype(bool))
+    env.close()
