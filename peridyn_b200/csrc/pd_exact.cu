@@ -33,8 +33,17 @@ __device__ __forceinline__ double mag3(double a1, double a2, double a3) {
     return sqrt(a1 * a1 + a2 * a2 + a3 * a3);
 }
 
-// One 256-bit load of a particle's record.
+// One 256-bit load of a particle's record.  The dependent kernels (pdl_enter)
+// are resident while the previous kernel on the stream still writes y, f and
+// mth.  They read those coherently (ld4) and behind the wait, take them
+// without __restrict__, and keep ld.global.nc (ld4_nc, __ldg) to data that is
+// complete since pd_env_finalize: x4, nbr.
 __device__ __forceinline__ double4 ld4(const double4 *p) {
+    double4 r;
+    asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ double4 ld4_nc(const double4 *p) {
     double4 r;
     asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
     return r;
@@ -326,8 +335,7 @@ __device__ __noinline__ double theta_term_general(double4 xp, double4 yp, double
 constexpr int32_t kThetaTile = 128;
 template <int NW>
 __global__ void __launch_bounds__(32 * NW, NW == 8 ? 3 : 1)
-    k_theta_slice(Geo g, const double4 *__restrict__ y, const uint32_t *__restrict__ win, double2 *__restrict__ mth,
-                  int64_t s0) {
+    k_theta_slice(Geo g, const double4 *y, const uint32_t *win, double2 *mth, int64_t s0) {
     __shared__ double term[kThetaTile][32];
     const int64_t s = s0 + blockIdx.x;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -337,7 +345,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 3 : 1)
     const int kind = tb >= 0 ? g.blocks[tb >> 8].kind : PD_MAT_SKIP;
     const int32_t n = g.cnt[p];
     const int32_t own = lane_record((int32_t)p, ti);
-    const double4 xp = ld4(g.x4 + own);
+    const double4 xp = ld4_nc(g.x4 + own);
     pdl_enter();  // before any return: the next kernel may wait for this one only
     if ((kind != PD_MAT_ORDINARY_STATE_BASED && kind != PD_MAT_ELASTO_PLASTIC) || (g.stop && *g.stop)) return;
     const double4 yp = ld4(y + own);
@@ -368,7 +376,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 3 : 1)
             const bool la = ka < n && ((wi[32 * (ka >> 5)] >> (ka & 31)) & 1u);
             const bool lb = kb < n && ((wi[32 * (kb >> 5)] >> (kb & 31)) & 1u);
             const int32_t qa = slot_record(st, own, na, la), qb = slot_record(st, own, nb2, lb);
-            const double4 xa = ld4(g.x4 + qa), ya = ld4(y + qa), xb = ld4(g.x4 + qb), yb = ld4(y + qb);
+            const double4 xa = ld4_nc(g.x4 + qa), ya = ld4(y + qa), xb = ld4_nc(g.x4 + qb), yb = ld4(y + qb);
             double ta, tb2;
             const bool ea = evaluate(xa, ya, ta), eb = evaluate(xb, yb, tb2);
             if (la && !ea) ta = theta_term_general(xp, yp, xa, ya, c_i);
@@ -393,8 +401,8 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 3 : 1)
 template <int KIND>
 __device__ __forceinline__ bool bond_term(const Geo &g, const DevBlock &B, int tp,
                                           double4 xp, double4 yp, double2 mp, double rho_p,
-                                          int32_t q, const double4 *__restrict__ y,
-                                          const double2 *__restrict__ mth, double &t0,
+                                          int32_t q, const double4 *y,
+                                          const double2 *mth, double &t0,
                                           double &t1, double &t2) {
     double4 xq = g.x4[q], yq = y[q];
     double X1 = xq.x - xp.x, X2 = xq.y - xp.y, X3 = xq.z - xp.z;
@@ -460,7 +468,7 @@ __device__ __forceinline__ double ep_t(const PairParam &pp, double xij, double e
 // (own, slot k of p) or from q's visit to p.
 __device__ __forceinline__ bool bond_term_ep(const Geo &g, const DevBlock &B, int tp, int64_t p, double4 xp,
                                              double4 yp, double2 mp, double rho_p, int32_t q, int32_t k, bool own,
-                                             const double4 *__restrict__ y, const double2 *__restrict__ mth,
+                                             const double4 *y, const double2 *mth,
                                              double &t0, double &t1, double &t2) {
     double4 xq = g.x4[q], yq = y[q];
     double X1 = xq.x - xp.x, X2 = xq.y - xp.y, X3 = xq.z - xp.z;
@@ -561,10 +569,10 @@ __global__ void __launch_bounds__(kThreads)
 // ---------------------------------------------------------------------
 template <int KIND>
 __device__ void force_serial_particle(const Geo &g, int64_t p, int32_t ti,
-                                      const double4 *__restrict__ y,
-                                      const double2 *__restrict__ mth,
-                                      const uint32_t *__restrict__ win,
-                                      uint32_t *__restrict__ wout, double4 *__restrict__ f,
+                                      const double4 *y,
+                                      const double2 *mth,
+                                      const uint32_t *win,
+                                      uint32_t *wout, double4 *f,
                                       int accumulate) {
     const DevBlock &B = g.blocks[ti >> 8];
     int tp = ti & 255;
@@ -704,7 +712,7 @@ inline size_t force_slice_bytes(int32_t cap) { return 768 * (size_t)cap + 128 * 
 // A bond the branch-free evaluation does not cover, with the operators.
 template <int KIND>
 __device__ __noinline__ bool bond_term_general(const Geo &g, const DevBlock &B, int64_t p, int tp, int32_t q,
-                                               const double4 *__restrict__ y, const double2 *__restrict__ mth,
+                                               const double4 *y, const double2 *mth,
                                                double *t) {
     return bond_term<KIND>(g, B, tp, g.x4[p], y[p], KIND != PD_MAT_BOND_BASED ? mth[p] : make_double2(0.0, 0.0),
                            g.tdens[B.type_base + tp], q, y, mth, t[0], t[1], t[2]);
@@ -712,9 +720,9 @@ __device__ __noinline__ bool bond_term_general(const Geo &g, const DevBlock &B, 
 
 // A particle of a slice the block evaluation does not cover (accumulating).
 __device__ __noinline__ void force_particle_general(const Geo &g, int64_t p, int32_t ti, int kind,
-                                                    const double4 *__restrict__ y, const double2 *__restrict__ mth,
-                                                    const uint32_t *__restrict__ win, uint32_t *__restrict__ wout,
-                                                    double4 *__restrict__ f) {
+                                                    const double4 *y, const double2 *mth,
+                                                    const uint32_t *win, uint32_t *wout,
+                                                    double4 *f) {
     if (kind == PD_MAT_BOND_BASED) force_serial_particle<PD_MAT_BOND_BASED>(g, p, ti, y, mth, win, wout, f, 1);
     else force_serial_particle<PD_MAT_ORDINARY_STATE_BASED>(g, p, ti, y, mth, win, wout, f, 1);
 }
@@ -729,12 +737,12 @@ struct SlotIn {
 template <int KIND, bool MULTI, bool ST, int NW>
 __device__ __forceinline__ void evaluate_slice(const Geo &g, const DevBlock &B, const SliceInfo &d, int64_t p,
                                                int32_t ti, int32_t n, int32_t L, int w, int lane,
-                                               const double4 *__restrict__ y, const double2 *__restrict__ mth,
-                                               const uint32_t *__restrict__ win, double *term, uint32_t *brk) {
+                                               const double4 *y, const double2 *mth,
+                                               const uint32_t *win, double *term, uint32_t *brk) {
     constexpr bool PMB = KIND == PD_MAT_BOND_BASED;
     const int tp = ti >= 0 ? ti & 255 : 0;
     const int32_t own = lane_record((int32_t)p, ti);
-    const double4 xp = ld4(g.x4 + own), yp = ld4(y + own);
+    const double4 xp = ld4_nc(g.x4 + own), yp = ld4(y + own);
     const double2 mp = PMB ? make_double2(0.0, 0.0) : mth[own];
     const double rho_p = g.tdens[B.type_base + tp];
     const PairParam pp0 = g.pairs[B.pair_base + tp + tp * B.nt];
@@ -749,9 +757,9 @@ __device__ __forceinline__ void evaluate_slice(const Geo &g, const DevBlock &B, 
     auto entry = [&](int32_t k) { return __ldg(nb + (ST ? k : 32 * k)); };  // (a slice stores all its slots)
     auto load = [&](int32_t q) {
         SlotIn r;
-        r.x = ld4(g.x4 + q);
+        r.x = ld4_nc(g.x4 + q);
         r.y = ld4(y + q);
-        r.m = PMB ? make_double2(0.0, 0.0) : __ldg(mth + q);
+        r.m = PMB ? make_double2(0.0, 0.0) : mth[q];
         r.q = q;
         return r;
     };
@@ -836,8 +844,8 @@ __device__ __forceinline__ void evaluate_slice(const Geo &g, const DevBlock &B, 
 template <int KIND, int NW>
 __device__ __forceinline__ void evaluate_kind(const Geo &g, const DevBlock &B, const SliceInfo &d, int64_t p,
                                               int32_t ti, int32_t n, int32_t L, int w, int lane,
-                                              const double4 *__restrict__ y, const double2 *__restrict__ mth,
-                                              const uint32_t *__restrict__ win, double *term, uint32_t *brk) {
+                                              const double4 *y, const double2 *mth,
+                                              const uint32_t *win, double *term, uint32_t *brk) {
     if (d.mode == kStencil) {
         if (B.nt > 1) evaluate_slice<KIND, true, true, NW>(g, B, d, p, ti, n, L, w, lane, y, mth, win, term, brk);
         else evaluate_slice<KIND, false, true, NW>(g, B, d, p, ti, n, L, w, lane, y, mth, win, term, brk);
@@ -849,8 +857,8 @@ __device__ __forceinline__ void evaluate_kind(const Geo &g, const DevBlock &B, c
 
 template <int NW>
 __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 1)
-    k_force_slice(Geo g, const double4 *__restrict__ y, const double2 *__restrict__ mth,
-                  const uint32_t *__restrict__ win, uint32_t *__restrict__ wout, double4 *__restrict__ f,
+    k_force_slice(Geo g, const double4 *y, const double2 *mth,
+                  const uint32_t *win, uint32_t *wout, double4 *f,
                   int accumulate, int32_t cap, int64_t s0) {
     extern __shared__ double term[];  // [slot][component][lane], then the broken bits [word][lane]
     const int64_t s = s0 + blockIdx.x;
@@ -1038,8 +1046,8 @@ __global__ void k_bc_vel(BCDev bc, int dir, const double4 *__restrict__ y, doubl
 // and 19 with this one, a 40,000-particle bar with two conditions 143 and 120.
 template <bool POST, bool PRE>
 __global__ void __launch_bounds__(256)
-    k_advance(int64_t N, double c, double dt, const double4 *__restrict__ f, double4 *__restrict__ v,
-              double4 *__restrict__ y, const double *__restrict__ mass, double4 *__restrict__ p,
+    k_advance(int64_t N, double c, double dt, const double4 *f, double4 *v,
+              double4 *y, const double *__restrict__ mass, double4 *p,
               const __grid_constant__ FusedBCs b, int64_t ts) {
     const int64_t i = blockIdx.x * (int64_t)256 + threadIdx.x;
     pdl_enter();

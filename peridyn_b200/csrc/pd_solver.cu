@@ -136,9 +136,8 @@ struct QsState {
 // max|f| / max|dy| reductions of :204 and the convergence test: the last
 // block to arrive combines the blocks' maxima (exact in any order).
 __global__ void __launch_bounds__(256)
-    k_qs_apply(int64_t N, const int32_t *__restrict__ freem, const double4 *__restrict__ f,
-               double4 *__restrict__ opt, double4 *__restrict__ y, double lambda, double kk,
-               double ss, double a, double f_tol, double x_tol, double *__restrict__ partial, QsState *qs) {
+    k_qs_apply(int64_t N, const int32_t *freem, const double4 *f, double4 *opt, double4 *y, double lambda, double kk,
+               double ss, double a, double f_tol, double x_tol, double *partial, QsState *qs) {
     __shared__ double sf[8], sy[8];
     __shared__ bool last;
     pdl_enter();
