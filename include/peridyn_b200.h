@@ -342,9 +342,11 @@ PD_API pd_status pd_env_profile(pd_env *env, int32_t enable);
 PD_API pd_status pd_env_profile_read(pd_env *env, double *total_ms, int64_t *launches);
 /* Kernel shape of the throughput modes (extension): warps per 32-particle
  * slice (1, 2, 4, 8) and bonds in flight per thread (FP32C: 2 or 4, FP64:
- * 1 or 2).  (0, 0) returns to the autotuner, which times every shape on
- * the first step -- for up to 65,536 particles also 16 warps per slice --
- * and caches the fastest per problem size. */
+ * 1 or 2); for up to 65,536 particles also 16 warps with the larger number
+ * of bonds in flight (with elasto-plastic blocks: the smaller).  (0, 0)
+ * returns to the autotuner, which times every shape on the first step and
+ * caches the fastest per problem size; pd_env_kernel_shape returns a shape
+ * this call accepts for an environment of the same blocks. */
 PD_API pd_status pd_env_set_kernel_shape(pd_env *env, int32_t warps_per_slice, int32_t unroll);
 /* The shape the throughput path runs with (after autotuning); (0, 0)
  * before the first throughput-mode step or in the serial mode. */
