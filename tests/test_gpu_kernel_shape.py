@@ -1,6 +1,10 @@
 """Kernel shapes of the throughput modes: the shape an environment was tuned to
 can be pinned on another one, the sixteen-warp shape only where the tuner may
-choose it."""
+choose it, and the tuner's cache keeps to that limit."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -56,3 +60,21 @@ def test_sixteen_warps_are_refused_above_the_limit():
     assert _abi.lib().pd_env_set_kernel_shape(env._h, 16, 4) == _abi.PD_ERR_ARG
     env.set_kernel_shape(8, 4)
     env.close()
+
+def test_tuned_shapes_are_not_shared_across_the_limit():
+    """65,600 and 65,536 particles lie in one class of sizes; only the smaller
+    body may run, and is timed with, sixteen warps per slice."""
+    code = ("import peridyn_b200 as pb\n"
+            "from peridyn_b200 import configs\n"
+            "for dims in ((41, 40, 40), (64, 32, 32)):\n"
+            "    w = configs.pmb_cube(dims=dims)\n"
+            "    env = pb.Env(1, w['materials'], [], [], w['dt'], precision='fp32c')\n"
+            "    pb.velocity_verlet_step(env, nsteps=2)\n")
+    env = dict(os.environ, PD_TUNE_LOG="1")
+    env.pop("PD_KERNEL_SHAPE", None)
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    lines = [s for s in r.stderr.splitlines() if s.startswith("pd autotune")]
+    assert [s.split()[2] for s in lines] == ["N=65600:", "N=65536:"]
+    assert " 16,4=" not in lines[0] and " 16,4=" in lines[1]
