@@ -2,6 +2,7 @@
 // device memory ownership, family construction and the solver sequencing of
 // src/solvers/*.jl on one CUDA stream.
 #include <algorithm>
+#include <climits>
 #include <chrono>
 #include <cmath>
 #include <cstdlib>
@@ -777,6 +778,35 @@ static pd_status build_runtime_layout_device(pd_env *env, const std::vector<int6
 // finalize: layout, upload, families, weighted volume, intact0
 // ---------------------------------------------------------------------
 
+// Unit of the FP64 throughput records.  Their walk takes a bond's reciprocal
+// weight as one inverse root of a sixth power of lengths, which is normal for
+// lengths within 2^170 (1e51) of one either way.  Environments whose bonds
+// are longer than 2^100 or shorter than 2^-100 are therefore held in a power
+// of two near them (an exact change of unit), the others as they are.
+// Bonds are no longer than the horizon (unless the host gave the family) and
+// the block's extent.
+static double bond_unit(const std::vector<HostBlock> &hb) {
+    int lo = INT_MAX, hi = INT_MIN;
+    for (const auto &b : hb) {
+        if (b.kind == PD_MAT_SKIP || b.n < 2) continue;
+        double len = 0.0;
+        for (int d = 0; d < 3; ++d) {
+            double mn = b.x[d], mx = b.x[d];
+            for (int64_t i = 1; i < b.n; ++i) {
+                mn = std::min(mn, b.x[3 * i + d]);
+                mx = std::max(mx, b.x[3 * i + d]);
+            }
+            len = std::max(len, mx - mn);
+        }
+        if (!b.host_family) len = std::min(len, b.horizon);
+        if (!(len > 0.0) || !std::isfinite(len)) continue;
+        lo = std::min(lo, std::ilogb(len));
+        hi = std::max(hi, std::ilogb(len));
+    }
+    if (lo > hi || (lo >= -100 && hi <= 100)) return 1.0;
+    return std::ldexp(1.0, -std::max(-1000, std::min(1000, lo + (hi - lo) / 2)));
+}
+
 extern "C" pd_status pd_env_finalize(pd_env *env) {
     PD_TRY(check_env(env));
     if (env->finalized) return fail(PD_ERR_STATE, "environment already finalized");
@@ -786,6 +816,7 @@ extern "C" pd_status pd_env_finalize(pd_env *env) {
     SetupClock clk;
 
     // --- internal layout ---
+    if (env->precision == PD_PREC_FP64) env->unit = bond_unit(env->hb);
     int64_t N = 0;
     for (auto &b : env->hb) {
         b.first_int = N;

@@ -271,6 +271,9 @@ struct pd_env {
     cudaStream_t copy_st = nullptr;
 
     // fast (FP64 / FP32C) state; see pd_fast.cu
+    // FP64 records: power of two times the bonds' lengths is near one (1 at
+    // ordinary lengths; see bond_unit)
+    double unit = 1.0;
     bool fast_valid = false;
     void *fast = nullptr;
     int shape = 0;  // fixed kernel shape 10 * warps_per_slice + unroll, 0 = autotune
