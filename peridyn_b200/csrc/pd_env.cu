@@ -87,10 +87,6 @@ pd::Geo pd_env::geo() const {
     g.fam = fam.p;
     g.deformed = deformed.p;
     g.stop = nullptr;
-    g.max_slots = max_slots;
-    g.has_ep = 0;
-    for (const auto &b : hb)
-        if (b.kind == PD_MAT_ELASTO_PLASTIC) g.has_ep = 1;
     g.td2 = td2.p;
     g.edp_in = edp[ecur].p;
     g.edp_out = edp[1 - ecur].p;
@@ -659,7 +655,6 @@ static pd_status build_runtime_layout(pd_env *env, const std::vector<int64_t> &s
     env->cnt_h = cnt;
     env->nnz = (int64_t)kSlice * nwords;
     env->walked = walked_slots(env->cnt_h);
-    env->max_slots = env->cnt_h.empty() ? 0 : *std::max_element(env->cnt_h.begin(), env->cnt_h.end());
     env->nbr_len = nbr_len;
     env->stencil_slices = nst;
     cudaStream_t st = env->st;
@@ -768,7 +763,6 @@ static pd_status build_runtime_layout_device(pd_env *env, const std::vector<int6
     env->cnt_h = cnt_b;
     env->nnz = (int64_t)kSlice * nwords;
     env->walked = walked_slots(env->cnt_h);
-    env->max_slots = env->cnt_h.empty() ? 0 : *std::max_element(env->cnt_h.begin(), env->cnt_h.end());
     env->nbr_len = nbr_len;
     env->stencil_slices = nst;
     return PD_OK;
@@ -1174,6 +1168,19 @@ extern "C" pd_status pd_env_finalize(pd_env *env) {
         }
         env->bcs.push_back(std::move(d));
     }
+    for (auto &b : env->hb) {
+        int64_t walked = 0;
+        for (int64_t i = 0; i < b.n; i += kSlice) {
+            const auto c = env->cnt_h.begin() + b.first_int + i;
+            const int32_t most = *std::max_element(c, c + std::min<int64_t>(kSlice, b.n - i));
+            b.slots = std::max(b.slots, most);
+            walked += most;
+        }
+        const int64_t slices = (b.n + kSlice - 1) / kSlice;
+        b.mean_slots = slices > 0 ? (int32_t)((walked + slices - 1) / slices) : 0;
+    }
+    env->force_runs = serial_runs(env, 0, env->hb.size(), false);
+    env->theta_runs = serial_runs(env, 0, env->hb.size(), true);
     // membership bits and list places for the serial mode's fused integration
     if (env->precision == PD_PREC_FP64_SERIAL && !env->hbc.empty() && env->hbc.size() <= (size_t)kMaxFusedBC) {
         std::vector<uint8_t> bits(N, 0);

@@ -114,6 +114,8 @@ struct HostBlock {
     std::vector<int64_t> family;
     std::vector<uint8_t> intact;
     int64_t first_env = 0, first_int = 0;
+    int32_t slots = 0;       // largest slot count of its particles
+    int32_t mean_slots = 0;  // slots a slice walks, on average
     int64_t cell_part_off = 0;
 };
 
@@ -201,7 +203,6 @@ struct pd_env {
     std::vector<int32_t> cnt_h;
     int64_t nnz = 0;       // bond slots (bits per bit array)
     int64_t walked = 0;    // slots the walks visit: per slice 32 x its largest slot count
-    int32_t max_slots = 0; // largest slot count of a particle
     int64_t nbr_len = 0;   // entries of nbr[]
     int64_t stencil_slices = 0;
     // Record staging plans of stencil slices (throughput path): the
@@ -240,6 +241,8 @@ struct pd_env {
     pd::DBuf<uint8_t> bc_bits;
     pd::DBuf<int32_t> bc_rank;
     std::vector<int64_t> bc_rank_off, bc_rank_lo;
+    // serial mode: how the blocks' forces and dilatations are evaluated
+    std::vector<pd::SerialRun> force_runs, theta_runs;
     std::vector<pd::DevContact> contacts;
     int64_t contact_epoch = 0;  // incremented whenever the contact lists change
 
@@ -310,6 +313,8 @@ pd_status fast_land_flags(pd_env *env);
 // estimate from particle counts and family rows; for admission control).
 int64_t footprint_estimate(const pd_env *env);
 pd_status fast_update_acc(pd_env *env);
+// Runs of the blocks [b0, b1) for the force or the dilatation.
+std::vector<SerialRun> serial_runs(const pd_env *env, size_t b0, size_t b1, bool theta);
 // momentum: p = m v at the end; stop: see Geo::stop.
 pd_status update_acc_serial(pd_env *env, bool momentum = true, const int32_t *stop = nullptr);
 }  // namespace pd

@@ -325,6 +325,45 @@ __device__ __noinline__ double theta_term_general(double4 xp, double4 yp, double
     const double wi = 1.0 / xij;
     return c_i * wi * xij * e * xq.w;
 }
+// The branch-free evaluation; returns whether it is exact.
+__device__ __forceinline__ bool theta_slot(const double4 &xp, const double4 &yp, const double4 &xq, const double4 &yq,
+                                           double c_i, double &t) {
+    const double X1 = xq.x - xp.x, X2 = xq.y - xp.y, X3 = xq.z - xp.z;
+    const double Y1 = yq.x - yp.x, Y2 = yq.y - yp.y, Y3 = yq.z - yp.z;
+    double xij, yij, rx, ry;
+    bool fast = sqrt_rcp_rn(X1 * X1 + X2 * X2 + X3 * X3, xij, rx);
+    fast = sqrt_rcp_rn(Y1 * Y1 + Y2 * Y2 + Y3 * Y3, yij, ry) && fast;
+    t = c_i * rx * xij * (yij - xij) * xq.w;
+    return fast;
+}
+
+// A thread per particle, one term after another: short slot lists on many
+// slices (serial_runs).  Bound by the latency of a term's roots.
+__global__ void __launch_bounds__(kThreads)
+    k_theta_serial(Geo g, const double4 *y, const uint32_t *win, double2 *mth, int64_t p0, int64_t p1) {
+    const int64_t p = p0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (p >= p1 || (g.stop && *g.stop)) return;
+    const int32_t ti = g.tinfo[p];
+    if (ti < 0) return;
+    const int kind = g.blocks[ti >> 8].kind;
+    if (kind != PD_MAT_ORDINARY_STATE_BASED && kind != PD_MAT_ELASTO_PLASTIC) return;
+    const double4 xp = g.x4[p], yp = y[p];
+    const double c_i = 3.0 / mth[p].x;
+    const int32_t n = g.cnt[p];
+    const BondRef br = bond_ref(g.si, g.nbr, win, p);
+    double th = 0.0;
+    uint32_t w = 0;
+    for (int32_t k = 0; k < n; ++k) {
+        if ((k & 31) == 0) w = *br.word(k);
+        if (!((w >> (k & 31)) & 1u)) continue;
+        const int32_t q = br.q(k);
+        const double4 xq = ld4_nc(g.x4 + q), yq = ld4(y + q);
+        double t;
+        if (!theta_slot(xp, yp, xq, yq, c_i, t)) t = theta_term_general(xp, yp, xq, yq, c_i);
+        th = th + t;
+    }
+    mth[p].y = th;
+}
 
 // One block per slice: the warps evaluate the terms of the slice's slots
 // side by side (tiles of kThetaTile slots in shared memory, a contiguous run
@@ -356,15 +395,6 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 3 : 1)
     const int32_t *nb = g.nbr + d.nbr + (st ? 0 : lane);
     const uint32_t *wi = win + d.word + lane;
     auto entry = [&](int32_t k) { return __ldg(nb + (st ? k : 32 * k)); };  // (a slice stores all its slots)
-    auto evaluate = [&](const double4 &xq, const double4 &yq, double &t) -> bool {
-        const double X1 = xq.x - xp.x, X2 = xq.y - xp.y, X3 = xq.z - xp.z;
-        const double Y1 = yq.x - yp.x, Y2 = yq.y - yp.y, Y3 = yq.z - yp.z;
-        double xij, yij, rx, ry;
-        bool fast = sqrt_rcp_rn(X1 * X1 + X2 * X2 + X3 * X3, xij, rx);
-        fast = sqrt_rcp_rn(Y1 * Y1 + Y2 * Y2 + Y3 * Y3, yij, ry) && fast;
-        t = c_i * rx * xij * (yij - xij) * xq.w;
-        return fast;
-    };
     double th = 0.0;
     for (int32_t base = 0; base < L; base += kThetaTile) {
         const int32_t m = min(kThetaTile, L - base);
@@ -378,7 +408,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 3 : 1)
             const int32_t qa = slot_record(st, own, na, la), qb = slot_record(st, own, nb2, lb);
             const double4 xa = ld4_nc(g.x4 + qa), ya = ld4(y + qa), xb = ld4_nc(g.x4 + qb), yb = ld4(y + qb);
             double ta, tb2;
-            const bool ea = evaluate(xa, ya, ta), eb = evaluate(xb, yb, tb2);
+            const bool ea = theta_slot(xp, yp, xa, ya, c_i, ta), eb = theta_slot(xp, yp, xb, yb, c_i, tb2);
             if (la && !ea) ta = theta_term_general(xp, yp, xa, ya, c_i);
             if (lb && !eb) tb2 = theta_term_general(xp, yp, xb, yb, c_i);
             term[j][lane] = la ? ta : 0.0;
@@ -429,6 +459,97 @@ __device__ __forceinline__ bool bond_term(const Geo &g, const DevBlock &B, int t
     t1 = xx * Y2 * xq.w / rho_p;
     t2 = xx * Y3 * xq.w / rho_p;
     return true;
+}
+
+// The same in branch-free arithmetic (pd_ieee.h).
+// What a particle's terms share.
+struct OwnTerm {
+    double4 x, y;
+    double2 m;
+    double rho, rrho, rm;  // rrho = 1 / rho, rm = 1 / m.x
+    bool ok;               // rho, m.x and c11 are within div_ok's range
+};
+// What a slot's evaluation needs of its neighbour.
+struct SlotIn {
+    double4 x, y;
+    double2 m;
+    int32_t q;
+};
+
+template <int KIND>
+__device__ __forceinline__ OwnTerm own_term(double4 x, double4 y, double2 m, double rho, double c11) {
+    constexpr bool PMB = KIND == PD_MAT_BOND_BASED;
+    return OwnTerm{x, y, m, rho, rcp_rn(rho), PMB ? 0.0 : rcp_rn(m.x),
+                   div_ok(rho) && (PMB ? div_ok(fabs(c11)) : div_ok(m.x))};
+}
+
+// The slot's term (zero unless live and within the critical stretch);
+// returns whether the evaluation is exact.  The numerators: ext is zero
+// or at least 2^-54 of the lengths, and so is s, at most 2^200; PMB: c in
+// [2^-100, 2^100) then keeps 0.5 t in range, LPS checks it; V < 2^100
+// bounds the last three from above.
+template <int KIND>
+__device__ __forceinline__ bool slot_term(const OwnTerm &o, double c11, const SlotIn &r, const PairParam &pp, bool live,
+                                          double &o0, double &o1, double &o2, bool &within) {
+    constexpr bool PMB = KIND == PD_MAT_BOND_BASED;
+    const double Y1 = r.y.x - o.y.x, Y2 = r.y.y - o.y.y, Y3 = r.y.z - o.y.z;
+    const double X1 = r.x.x - o.x.x, X2 = r.x.y - o.x.y, X3 = r.x.z - o.x.z;
+    double xij, yij, rx, ry;
+    bool fast = sqrt_rcp_rn(X1 * X1 + X2 * X2 + X3 * X3, xij, rx) && o.ok;
+    fast = sqrt_rcp_rn(Y1 * Y1 + Y2 * Y2 + Y3 * Y3, yij, ry) && fast;
+    fast = (uint32_t)hi_word(r.x.w) < ((1023u + 100u) << 20) && fast;
+    const double ext = yij - xij;
+    const double s = div_rn(ext, xij, rx);
+    within = s < pp.cs;
+    double t;
+    if (PMB) {
+        t = s * c11;
+    } else {
+        fast = fast && div_ok(r.m.x);
+        const double a = div_rn(rx, o.m.x, o.rm), b = div_rn(rx, r.m.x, rcp_rn(r.m.x));
+        t = pp.k35 * (o.m.y * xij * a + r.m.y * xij * b) + pp.g15 * ext * (a + b);
+    }
+    const double ht = 0.5 * t;
+    if (!PMB) fast = fast && magnitude(ht) >= kMagLo && (2u * (uint32_t)hi_word(ht)) < kMagHi;
+    double xx = div_rn(ht, yij, ry);
+    xx = live && within ? xx : 0.0;
+    o0 = xx * Y1 * r.x.w;
+    o1 = xx * Y2 * r.x.w;
+    o2 = xx * Y3 * r.x.w;
+    fast = fast && min(min(magnitude(o0), magnitude(o1)), magnitude(o2)) >= kMagLo;
+    o0 = div_rn(o0, o.rho, o.rrho);
+    o1 = div_rn(o1, o.rho, o.rrho);
+    o2 = div_rn(o2, o.rho, o.rrho);
+    return fast;
+}
+
+// A bond the branch-free evaluation does not cover, with the operators.
+template <int KIND>
+__device__ __noinline__ bool bond_term_general(const Geo &g, const DevBlock &B, int64_t p, int tp, int32_t q,
+                                               const double4 *y, const double2 *mth, double *t) {
+    return bond_term<KIND>(g, B, tp, g.x4[p], y[p], KIND != PD_MAT_BOND_BASED ? mth[p] : make_double2(0.0, 0.0),
+                           g.tdens[B.type_base + tp], q, y, mth, t[0], t[1], t[2]);
+}
+
+// bond_term by the branch-free evaluation where it is exact.
+template <int KIND>
+__device__ __forceinline__ bool bond_term_fast(const Geo &g, const DevBlock &B, int64_t p, int tp, const OwnTerm &o,
+                                               int32_t q, const double4 *y, const double2 *mth, double &t0, double &t1,
+                                               double &t2) {
+    SlotIn r;
+    r.x = ld4_nc(g.x4 + q);
+    r.y = ld4(y + q);
+    r.m = KIND == PD_MAT_BOND_BASED ? make_double2(0.0, 0.0) : mth[q];
+    r.q = q;
+    const int tq = B.nt > 1 ? (g.tinfo[q] & 255) : 0;
+    bool within;
+    if (slot_term<KIND>(o, B.c11, r, g.pairs[B.pair_base + tp + tq * B.nt], true, t0, t1, t2, within)) return within;
+    double t[3] = {0.0, 0.0, 0.0};
+    within = bond_term_general<KIND>(g, B, p, tp, q, y, mth, t);
+    t0 = t[0];
+    t1 = t[1];
+    t2 = t[2];
+    return within;
 }
 
 // ---------------------------------------------------------------------
@@ -580,6 +701,7 @@ __device__ void force_serial_particle(const Geo &g, int64_t p, int32_t ti,
     double2 mp = KIND != PD_MAT_BOND_BASED ? mth[p] : make_double2(0.0, 0.0);
     constexpr bool EP = KIND == PD_MAT_ELASTO_PLASTIC;
     double rho_p = g.tdens[B.type_base + tp];
+    const OwnTerm o = own_term<EP ? PD_MAT_BOND_BASED : KIND>(xp, yp, mp, rho_p, B.c11);
     int32_t n = g.cnt[p];
     const BondRef br = bond_ref(g.si, g.nbr, win, p);
     uint32_t *wo = wout + g.si[p >> 5].word + (p & 31);
@@ -599,7 +721,7 @@ __device__ void force_serial_particle(const Geo &g, int64_t p, int32_t ti,
         uint32_t w = *br.word(k);
         if (!((w >> (k & 31)) & 1u)) continue;
         if (EP ? bond_term_ep(g, B, tp, p, xp, yp, mp, rho_p, q, k, false, y, mth, t0, t1, t2)
-               : bond_term<KIND>(g, B, tp, xp, yp, mp, rho_p, q, y, mth, t0, t1, t2)) {
+               : bond_term_fast<EP ? PD_MAT_BOND_BASED : KIND>(g, B, p, tp, o, q, y, mth, t0, t1, t2)) {
             fx = fx + t0;
             fy = fy + t1;
             fz = fz + t2;
@@ -620,7 +742,7 @@ __device__ void force_serial_particle(const Geo &g, int64_t p, int32_t ti,
         if (!((w >> (k & 31)) & 1u)) continue;
         int32_t q = br.q(k);
         if (EP ? bond_term_ep(g, B, tp, p, xp, yp, mp, rho_p, q, k, true, y, mth, t0, t1, t2)
-               : bond_term<KIND>(g, B, tp, xp, yp, mp, rho_p, q, y, mth, t0, t1, t2)) {
+               : bond_term_fast<EP ? PD_MAT_BOND_BASED : KIND>(g, B, p, tp, o, q, y, mth, t0, t1, t2)) {
             fx = fx + t0;
             fy = fy + t1;
             fz = fz + t2;
@@ -635,7 +757,7 @@ __device__ void force_serial_particle(const Geo &g, int64_t p, int32_t ti,
         uint32_t ww = *br.word(k);
         if (!((ww >> (k & 31)) & 1u)) continue;
         if (EP ? bond_term_ep(g, B, tp, p, xp, yp, mp, rho_p, q, k, false, y, mth, t0, t1, t2)
-               : bond_term<KIND>(g, B, tp, xp, yp, mp, rho_p, q, y, mth, t0, t1, t2)) {
+               : bond_term_fast<EP ? PD_MAT_BOND_BASED : KIND>(g, B, p, tp, o, q, y, mth, t0, t1, t2)) {
             fx = fx + t0;
             fy = fy + t1;
             fz = fz + t2;
@@ -647,9 +769,14 @@ __device__ void force_serial_particle(const Geo &g, int64_t p, int32_t ti,
 // The slots a 32-particle slice walks: the largest slot count of its lanes.
 __device__ __forceinline__ int32_t slice_slots(int32_t n) { return (int32_t)__reduce_max_sync(0xffffffffu, (unsigned)n); }
 
-// One thread per particle, every bond evaluated from both visits: the
-// elasto-plastic blocks (whose two visits differ) and slices with more than
-// cap slots.  The other slices belong to k_force_slice.
+// One thread per particle, every bond evaluated from both visits: short slot
+// lists on many slices (serial_runs; cap < 0: all of the range), and of the
+// rest the elasto-plastic blocks (whose two visits differ) and slices with
+// more than cap slots.  The other slices belong to k_force_slice.  Bound by
+// the latency of a bond's roots and quotients, which it meets twice per slot
+// in a row; branch-free as in k_force_slice (8,000 particles with 304 slots:
+// 338 us per evaluation, 454 with the operators; 262,144 with 18 slots, most
+// of them undisturbed: 108 against 249 us per step).
 __global__ void __launch_bounds__(kThreads)
     k_force_serial(Geo g, const double4 *__restrict__ y, const double2 *__restrict__ mth,
                    const uint32_t *__restrict__ win, uint32_t *__restrict__ wout,
@@ -709,15 +836,6 @@ constexpr int32_t kForceSlots = 288;
 constexpr int64_t kWideSlices = 148;  // SMs of a B200
 inline size_t force_slice_bytes(int32_t cap) { return 768 * (size_t)cap + 128 * (size_t)((cap + 31) / 32); }
 
-// A bond the branch-free evaluation does not cover, with the operators.
-template <int KIND>
-__device__ __noinline__ bool bond_term_general(const Geo &g, const DevBlock &B, int64_t p, int tp, int32_t q,
-                                               const double4 *y, const double2 *mth,
-                                               double *t) {
-    return bond_term<KIND>(g, B, tp, g.x4[p], y[p], KIND != PD_MAT_BOND_BASED ? mth[p] : make_double2(0.0, 0.0),
-                           g.tdens[B.type_base + tp], q, y, mth, t[0], t[1], t[2]);
-}
-
 // A particle of a slice the block evaluation does not cover (accumulating).
 __device__ __noinline__ void force_particle_general(const Geo &g, int64_t p, int32_t ti, int kind,
                                                     const double4 *y, const double2 *mth,
@@ -727,13 +845,6 @@ __device__ __noinline__ void force_particle_general(const Geo &g, int64_t p, int
     else force_serial_particle<PD_MAT_ORDINARY_STATE_BASED>(g, p, ti, y, mth, win, wout, f, 1);
 }
 
-// What a slot's evaluation needs of its neighbour.
-struct SlotIn {
-    double4 x, y;
-    double2 m;
-    int32_t q;
-};
-
 template <int KIND, bool MULTI, bool ST, int NW>
 __device__ __forceinline__ void evaluate_slice(const Geo &g, const DevBlock &B, const SliceInfo &d, int64_t p,
                                                int32_t ti, int32_t n, int32_t L, int w, int lane,
@@ -742,13 +853,10 @@ __device__ __forceinline__ void evaluate_slice(const Geo &g, const DevBlock &B, 
     constexpr bool PMB = KIND == PD_MAT_BOND_BASED;
     const int tp = ti >= 0 ? ti & 255 : 0;
     const int32_t own = lane_record((int32_t)p, ti);
-    const double4 xp = ld4_nc(g.x4 + own), yp = ld4(y + own);
-    const double2 mp = PMB ? make_double2(0.0, 0.0) : mth[own];
-    const double rho_p = g.tdens[B.type_base + tp];
     const PairParam pp0 = g.pairs[B.pair_base + tp + tp * B.nt];
     const double c11 = B.c11;
-    const bool own_ok = div_ok(rho_p) && (PMB ? div_ok(fabs(c11)) : div_ok(mp.x));
-    const double rrho = rcp_rn(rho_p), rmp = PMB ? 0.0 : rcp_rn(mp.x);
+    const OwnTerm o = own_term<KIND>(ld4_nc(g.x4 + own), ld4(y + own), PMB ? make_double2(0.0, 0.0) : mth[own],
+                                     g.tdens[B.type_base + tp], c11);
     const int32_t *nb = g.nbr + d.nbr + (ST ? 0 : lane);
     const uint32_t *wi = win + d.word + lane;
     // warp w evaluates the contiguous slots [k0, k1)
@@ -763,42 +871,8 @@ __device__ __forceinline__ void evaluate_slice(const Geo &g, const DevBlock &B, 
         r.q = q;
         return r;
     };
-    // The slot's term (zero unless live and within the critical stretch);
-    // returns whether the evaluation is exact.  The numerators: ext is zero
-    // or at least 2^-54 of the lengths, and so is s, at most 2^200; PMB: c in
-    // [2^-100, 2^100) then keeps 0.5 t in range, LPS checks it; V < 2^100
-    // bounds the last three from above.
-    auto evaluate = [&](const SlotIn &r, bool live, double &o0, double &o1, double &o2, bool &within) -> bool {
-        const double Y1 = r.y.x - yp.x, Y2 = r.y.y - yp.y, Y3 = r.y.z - yp.z;
-        const double X1 = r.x.x - xp.x, X2 = r.x.y - xp.y, X3 = r.x.z - xp.z;
-        double xij, yij, rx, ry;
-        bool fast = sqrt_rcp_rn(X1 * X1 + X2 * X2 + X3 * X3, xij, rx) && own_ok;
-        fast = sqrt_rcp_rn(Y1 * Y1 + Y2 * Y2 + Y3 * Y3, yij, ry) && fast;
-        fast = (uint32_t)hi_word(r.x.w) < ((1023u + 100u) << 20) && fast;
-        const PairParam pp = MULTI ? g.pairs[slot_pair(B.pair_base, B.nt, tp, g.tinfo[r.q], live)] : pp0;
-        const double ext = yij - xij;
-        const double s = div_rn(ext, xij, rx);
-        within = s < pp.cs;
-        double t;
-        if (PMB) {
-            t = s * c11;
-        } else {
-            fast = fast && div_ok(r.m.x);
-            const double a = div_rn(rx, mp.x, rmp), b = div_rn(rx, r.m.x, rcp_rn(r.m.x));
-            t = pp.k35 * (mp.y * xij * a + r.m.y * xij * b) + pp.g15 * ext * (a + b);
-        }
-        const double ht = 0.5 * t;
-        if (!PMB) fast = fast && magnitude(ht) >= kMagLo && (2u * (uint32_t)hi_word(ht)) < kMagHi;
-        double xx = div_rn(ht, yij, ry);
-        xx = live && within ? xx : 0.0;
-        o0 = xx * Y1 * r.x.w;
-        o1 = xx * Y2 * r.x.w;
-        o2 = xx * Y3 * r.x.w;
-        fast = fast && min(min(magnitude(o0), magnitude(o1)), magnitude(o2)) >= kMagLo;
-        o0 = div_rn(o0, rho_p, rrho);
-        o1 = div_rn(o1, rho_p, rrho);
-        o2 = div_rn(o2, rho_p, rrho);
-        return fast;
+    auto pair = [&](const SlotIn &r, bool live) {
+        return MULTI ? g.pairs[slot_pair(B.pair_base, B.nt, tp, g.tinfo[r.q], live)] : pp0;
     };
     uint32_t bits = 0, gone = 0;
     auto finish = [&](int32_t k, int32_t q, bool live, bool exact, bool within, double o0, double o1, double o2) {
@@ -832,7 +906,8 @@ __device__ __forceinline__ void evaluate_slice(const Geo &g, const DevBlock &B, 
             nb2 = entry(min(next + 1, k1 - 1));
             double a0, a1, a2, b0, b1, bz;
             bool wa, wb;
-            const bool ea = evaluate(ra, la, a0, a1, a2, wa), eb = evaluate(rb, lb, b0, b1, bz, wb);
+            const bool ea = slot_term<KIND>(o, c11, ra, pair(ra, la), la, a0, a1, a2, wa);
+            const bool eb = slot_term<KIND>(o, c11, rb, pair(rb, lb), lb, b0, b1, bz, wb);
             finish(k, ra.q, la, ea, wa, a0, a1, a2);
             if (two) finish(k + 1, rb.q, lb, eb, wb, b0, b1, bz);
         }
@@ -1346,12 +1421,14 @@ void launch_weighted_volume(cudaStream_t st, const Geo &g, double2 *mth) {
 static bool wide_slices(int64_t slices) { return slices <= kWideSlices; }
 
 void launch_theta_serial(cudaStream_t st, const Geo &g, const double4 *y, const uint32_t *win,
-                         double2 *mth, int64_t p0, int64_t p1) {
-    if (p1 <= p0) return;
-    const int64_t S = (p1 - p0) / 32;
-    if (wide_slices(S)) launch_dep(k_theta_slice<16>, (unsigned)S, 512, st, g, y, win, mth, p0 / 32);
-    else launch_dep(k_theta_slice<8>, (unsigned)S, 256, st, g, y, win, mth, p0 / 32);
-    pd::note_launch();
+                         double2 *mth, const SerialRun *runs, size_t n_runs) {
+    for (const SerialRun *r = runs; r < runs + n_runs; ++r) {
+        const int64_t S = (r->p1 - r->p0) / 32;
+        if (!r->by_slice) k_theta_serial<<<grid_for(r->p1 - r->p0), kThreads, 0, st>>>(g, y, win, mth, r->p0, r->p1);
+        else if (wide_slices(S)) launch_dep(k_theta_slice<16>, (unsigned)S, 512, st, g, y, win, mth, r->p0 / 32);
+        else launch_dep(k_theta_slice<8>, (unsigned)S, 256, st, g, y, win, mth, r->p0 / 32);
+        pd::note_launch();
+    }
 }
 
 void launch_td_serial(cudaStream_t st, const Geo &g, const double4 *y, const double2 *mth,
@@ -1376,20 +1453,26 @@ static void force_slice_attrs() {
 
 void launch_force_serial(cudaStream_t st, const Geo &g, const double4 *y, const double2 *mth,
                          const uint32_t *win, uint32_t *wout, double4 *f, int accumulate,
-                         int64_t p0, int64_t p1) {
-    if (p1 <= p0) return;
-    const int32_t cap = g.max_slots < kForceSlots ? g.max_slots : kForceSlots;
-    const size_t sm = force_slice_bytes(cap);
-    const int64_t S = (p1 - p0) / 32;
-    force_slice_attrs();
-    if (wide_slices(S))
-        launch_dep_smem(k_force_slice<16>, (unsigned)S, 512, sm, st, g, y, mth, win, wout, f, accumulate, cap, p0 / 32);
-    else
-        launch_dep_smem(k_force_slice<8>, (unsigned)S, 256, sm, st, g, y, mth, win, wout, f, accumulate, cap, p0 / 32);
-    pd::note_launch();
-    if (g.has_ep || g.max_slots > cap) {
-        k_force_serial<<<grid_for(p1 - p0), kThreads, 0, st>>>(g, y, mth, win, wout, f, accumulate, cap, p0, p1);
-        pd::note_launch();
+                         const SerialRun *runs, size_t n_runs) {
+    for (const SerialRun *r = runs; r < runs + n_runs; ++r) {
+        const int32_t cap = !r->by_slice ? -1 : r->slots < kForceSlots ? r->slots : kForceSlots;
+        const int64_t S = (r->p1 - r->p0) / 32;
+        if (r->by_slice) {
+            const size_t sm = force_slice_bytes(cap);
+            force_slice_attrs();
+            if (wide_slices(S))
+                launch_dep_smem(k_force_slice<16>, (unsigned)S, 512, sm, st, g, y, mth, win, wout, f, accumulate, cap,
+                                r->p0 / 32);
+            else
+                launch_dep_smem(k_force_slice<8>, (unsigned)S, 256, sm, st, g, y, mth, win, wout, f, accumulate, cap,
+                                r->p0 / 32);
+            pd::note_launch();
+        }
+        if (r->ep || r->slots > cap) {
+            k_force_serial<<<grid_for(r->p1 - r->p0), kThreads, 0, st>>>(g, y, mth, win, wout, f, accumulate, cap,
+                                                                         r->p0, r->p1);
+            pd::note_launch();
+        }
     }
 }
 

@@ -117,8 +117,6 @@ struct Geo {
     const int32_t *nbr;        // bond index data (see SliceInfo)
     const uint32_t *fam;       // family-member bits (same layout as intact)
     const int32_t *deformed;   // per block
-    int32_t max_slots;         // largest slot count of a particle
-    int32_t has_ep;            // some block is elasto-plastic
     const int32_t *stop;       // not null: the force kernels return at once when *stop is set
     // elasto-plastic blocks: td_norm2 per particle, plastic deviatoric
     // strain per bond slot (read from edp_in, written to edp_out)
@@ -203,11 +201,19 @@ void launch_popcount(cudaStream_t st, int64_t N, const SliceInfo *si, const int3
 void launch_weighted_volume(cudaStream_t st, const Geo &g, double2 *mth);
 
 // Serial-order FP64 force path.
+// Consecutive blocks that one kernel evaluates: a block of warps per slice,
+// or a thread per particle.
+struct SerialRun {
+    int64_t p0, p1;   // internal particle range (multiples of 32)
+    int32_t slots;    // largest slot count of its particles
+    bool by_slice;
+    bool ep;          // holds elasto-plastic blocks
+};
 void launch_theta_serial(cudaStream_t st, const Geo &g, const double4 *y, const uint32_t *win,
-                         double2 *mth, int64_t p0, int64_t p1);
+                         double2 *mth, const SerialRun *runs, size_t n_runs);
 void launch_force_serial(cudaStream_t st, const Geo &g, const double4 *y, const double2 *mth,
                          const uint32_t *win, uint32_t *wout, double4 *f, int accumulate,
-                         int64_t p0, int64_t p1);
+                         const SerialRun *runs, size_t n_runs);
 // elasto_plastic.jl:166-172 out_of_loop! td_norm2 pass (breaks bonds too)
 void launch_td_serial(cudaStream_t st, const Geo &g, const double4 *y, const double2 *mth,
                       const uint32_t *win, uint32_t *wout, int64_t p0, int64_t p1);

@@ -224,6 +224,59 @@ __global__ void k_clear_idx(int64_t n, const int32_t *__restrict__ idx, int32_t 
 
 namespace pd {
 
+// How the blocks [b0, b1) are evaluated.  A block of warps per slice
+// evaluates every bond once and side by side, but an SM holds two or three of
+// them, each some 4.5 us long however few its slots; a thread per particle
+// evaluates every bond at both visits, one after another.  Short slot lists
+// on many slices are therefore left to threads.  Steps of strained
+// bond-based cubes in us, threads / slices:
+//   slots         6          18           26           32          120
+//     250 slices  15 / 11    28 / 12      37 / 13      42 / 13     132 / 23
+//     686         17 / 18    30 / 22      40 / 23      44 / 23     147 / 47
+//   1,229         20 / 25    32 / 31      41 / 34      48 / 34     153 / 71
+//   2,000         21 / 37    38 / 45      50 / 48      59 / 49     198 / 108
+//   8,192         52 / 117   109 / 148    149 / 161    179 / 163   641 / 394
+//  65,536         364 / 1054 807 / 1290   1100 / 1390  1331 / 1395 4741 / 3231
+// The dilatation's blocks do less per slice and its line lies higher (32
+// slots, state-based step with the force by slices: 8,192 slices 228 with
+// threads, 256 without; 65,536: 1844 and 2265).  The elasto-plastic force,
+// whose two visits differ, has the thread form only.
+std::vector<SerialRun> serial_runs(const pd_env *env, size_t b0, size_t b1, bool theta) {
+    constexpr size_t kMaxRuns = 8;
+    auto takes = [&](const HostBlock &b) {
+        return !theta || b.kind == PD_MAT_ORDINARY_STATE_BASED || b.kind == PD_MAT_ELASTO_PLASTIC;
+    };
+    auto slices = [](const HostBlock &b) { return (b.n + kSlice - 1) / kSlice; };
+    int64_t S = 0, wide = 0;
+    for (size_t k = b0; k < b1; ++k)
+        if (takes(env->hb[k])) S += slices(env->hb[k]);
+    std::vector<SerialRun> runs;
+    for (size_t k = b0; k < b1; ++k) {
+        const HostBlock &b = env->hb[k];
+        if (!takes(b) || b.n == 0) continue;
+        const bool ep = b.kind == PD_MAT_ELASTO_PLASTIC;
+        const bool by_slice = (theta || !ep) && !(b.mean_slots <= (theta ? 40 : 28) && S >= 300 + 70 * (int64_t)b.mean_slots);
+        const int64_t p0 = b.first_int, p1 = p0 + kSlice * slices(b);
+        if (by_slice) wide += slices(b);
+        if (!runs.empty() && runs.back().p1 == p0 && runs.back().by_slice == by_slice) {
+            runs.back().p1 = p1;
+            runs.back().slots = std::max(runs.back().slots, b.slots);
+            runs.back().ep |= ep;
+        } else {
+            runs.push_back(SerialRun{p0, p1, b.slots, by_slice, ep});
+        }
+    }
+    if (runs.size() <= kMaxRuns) return runs;
+    // many alternating blocks: one launch over all of them (the kernels leave
+    // what they do not evaluate), in the form that suits more slices
+    SerialRun all{runs.front().p0, runs.back().p1, 0, 2 * wide >= S, false};
+    for (const auto &r : runs) {
+        all.slots = std::max(all.slots, r.slots);
+        all.ep |= r.ep;
+    }
+    return {all};
+}
+
 // update_acc! (solvers.jl:320-336) in serial-order FP64.
 pd_status update_acc_serial(pd_env *env, bool momentum, const int32_t *stop) {
     cudaStream_t st = env->st;
@@ -256,7 +309,11 @@ pd_status update_acc_serial(pd_env *env, bool momentum, const int32_t *stop) {
         any_lps |= hb.kind == PD_MAT_ORDINARY_STATE_BASED || hb.kind == PD_MAT_ELASTO_PLASTIC;
         any_ep |= hb.kind == PD_MAT_ELASTO_PLASTIC;
     }
-    if (any_lps) launch_theta_serial(st, g, env->y.p, env->words[env->cur].p, env->mth.p, 0, env->N);
+    if (any_lps)
+        launch_theta_serial(st, g, env->y.p, env->words[env->cur].p, env->mth.p, env->theta_runs.data(),
+                            env->theta_runs.size());
+    const SerialRun *runs = env->force_runs.data();
+    const size_t n_runs = env->force_runs.size();
     if (any_ep) {
         // elasto_plastic.jl:170-171: td_norm2 pass (breaks bonds), then the
         // bond loop on its flags, back into words[cur]; edp is double-buffered
@@ -264,14 +321,14 @@ pd_status update_acc_serial(pd_env *env, bool momentum, const int32_t *stop) {
                          env->N);
         prof_begin(env, st);
         launch_force_serial(st, g, env->y.p, env->mth.p, env->words[1 - env->cur].p, env->words[env->cur].p,
-                            env->f.p, 0, 0, env->N);
+                            env->f.p, 0, runs, n_runs);
         prof_end(env, st);
         env->ecur = 1 - env->ecur;
     } else {
         // fill!(f, 0) + force_density_T! for every block
         prof_begin(env, st);
         launch_force_serial(st, g, env->y.p, env->mth.p, env->words[env->cur].p, env->words[1 - env->cur].p,
-                            env->f.p, 0, 0, env->N);
+                            env->f.p, 0, runs, n_runs);
         prof_end(env, st);
         env->cur = 1 - env->cur;
     }
@@ -453,7 +510,8 @@ extern "C" pd_status pd_env_qsdrag(pd_env *env, double step_size, double drag, i
     QsState *qs = (QsState *)env->qs_state.p;
     CK(cudaMemsetAsync(qs, 0, sizeof(QsState), st));
     QsState h{};
-    const bool ep = env->geo().has_ep != 0;
+    bool ep = false;
+    for (const auto &b : env->hb) ep |= b.kind == PD_MAT_ELASTO_PLASTIC;
     for (int64_t batch = 2; h.iters < max_iter && !h.done; batch = std::min(2 * batch, kQsBatch)) {
         PD_TRY(refresh_deformed(env));
         bool known = env->hc.empty() && !env->prof;  // (profiling counts the iterations that run)
@@ -525,13 +583,14 @@ extern "C" pd_status pd_force_density_device(pd_env *env, int64_t block, double 
     launch_unpack3(st, hb.n, f_dev + 3 * hb.first_env, map, env->tmp_f.p);
     Geo g = env->geo();
     int64_t p0 = hb.first_int, p1 = hb.first_int + ((hb.n + 31) / 32) * 32;
+    const auto theta = serial_runs(env, block, block + 1, true), force = serial_runs(env, block, block + 1, false);
     if (hb.kind == PD_MAT_ORDINARY_STATE_BASED)
-        launch_theta_serial(st, g, env->tmp_y.p, env->words[env->cur].p, env->mth.p, p0, p1);
+        launch_theta_serial(st, g, env->tmp_y.p, env->words[env->cur].p, env->mth.p, theta.data(), theta.size());
     // force_density_T! itself has no gate: compute unconditionally
     std::vector<int32_t> one(1, 1);
     CK(cudaMemcpyAsync(env->deformed.p + block, one.data(), 4, cudaMemcpyHostToDevice, st));
     launch_force_serial(st, g, env->tmp_y.p, env->mth.p, env->words[env->cur].p, env->words[1 - env->cur].p,
-                        env->tmp_f.p, 1, p0, p1);
+                        env->tmp_f.p, 1, force.data(), force.size());
     int64_t w0 = env->sinfo_h[p0 / 32].word, w1 = env->sinfo_h[p1 / 32].word;
     if (w1 > w0)
         CK(cudaMemcpyAsync(env->words[env->cur].p + w0, env->words[1 - env->cur].p + w0, (w1 - w0) * 4,

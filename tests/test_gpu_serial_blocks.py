@@ -22,6 +22,9 @@ def block(law, dims, ntypes, first_type, offset, factor=2.3, seed=5):
     r = np.linspace(1.0, 1.2, pairs)
     rho = list(np.linspace(2000.0, 2600.0, ntypes))
     cs = list(0.003 * r)
+    if law == "ep":
+        return pb.PeridynamicsMaterial(gen, pb.ElastoPlasticSolidSpecific(list(46.7e9 * r), list(28e9 * r), cs, rho,
+                                                                          list(2e7 * r)))
     if law == "pmb":
         return pb.PeridynamicsMaterial(gen, pb.BondBasedSpecific(list(14.9e9 * r), cs, rho))
     return pb.PeridynamicsMaterial(gen, pb.OrdinaryStateBasedSpecific(list(20e9 * r), list(9e9 * r), cs, rho))
@@ -84,4 +87,46 @@ def test_one_block_of_several_through_device_pointers(oracle, law, entry):
         assert np.array_equal(f[:, own], ora.f[:, own])
         assert np.array_equal(np.delete(f, np.r_[own], axis=1), np.delete(f0, np.r_[own], axis=1))
         assert np.array_equal(env._family(b)[1], B.intact.astype(bool))
+    env.close()
+
+
+@pytest.mark.parametrize("law", ["pmb", "lps"])
+@pytest.mark.parametrize("factor,dims", [(1.1, (36, 32, 32)),   # 6 slots, 1152 slices: threads
+                                         (1.1, (24, 25, 24)),   # 450 slices: warps per slice
+                                         (1.5, (46, 42, 40)),   # 18 slots, 2415 slices: threads
+                                         (2.1, (52, 51, 46))])  # 32 slots, 3812 slices: dilatation by threads
+def test_short_slot_lists_on_many_slices(oracle, law, factor, dims):
+    """A thread per particle or a block per slice: the same numbers."""
+    m = block(law, dims, 2, 1, 0.0, factor=factor)
+    env = pb.Env(1, [m], [], [], 2.0e-8)
+    ora = oracle.OracleEnv([m], [], [], 2.0e-8)
+    pb.velocity_verlet_step(env, nsteps=6)
+    for _ in range(6):
+        ora.vv_step()
+    y, v, f, _ = env.get_state()
+    assert np.array_equal(f, ora.f)
+    assert np.array_equal(v, ora.v)
+    assert np.array_equal(y, ora.y)
+    assert np.array_equal(env._family(0)[1], ora.blocks[0].intact.astype(bool))
+    env.close()
+
+
+@pytest.mark.parametrize("larger", ["ep", "others"])
+def test_many_alternating_blocks(oracle, larger):
+    """More runs of blocks than are launched one by one (the elasto-plastic
+    force has the thread form only): one launch in the form of the larger part."""
+    mats, t = [], 1
+    for k in range(12):
+        law, nt = ("ep", "pmb", "ep", "lps")[k % 4], 1 + k % 3
+        n = 6 if (law == "ep") == (larger == "ep") else 3
+        mats.append(block(law, (4 + k % 4, n, 3), nt, t, 0.02 * k, seed=k))
+        t += nt
+    env = pb.Env(1, mats, [], [], 2.0e-8)
+    ora = oracle.OracleEnv(mats, [], [], 2.0e-8)
+    pb.velocity_verlet_step(env, nsteps=10)
+    for _ in range(10):
+        ora.vv_step()
+    y, v, f, _ = env.get_state()
+    assert np.array_equal(f, ora.f)
+    assert np.array_equal(y, ora.y)
     env.close()
