@@ -930,33 +930,54 @@ __device__ __forceinline__ void evaluate_kind(const Geo &g, const DevBlock &B, c
     }
 }
 
-template <int NW>
-__global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 1)
-    k_force_slice(Geo g, const double4 *y, const double2 *mth,
-                  const uint32_t *win, uint32_t *wout, double4 *f,
-                  int accumulate, int32_t cap, int64_t s0) {
-    extern __shared__ double term[];  // [slot][component][lane], then the broken bits [word][lane]
-    const int64_t s = s0 + blockIdx.x;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t p = 32 * s + lane;
-    const int32_t ti = g.tinfo[p], n = g.cnt[p];
-    const SliceInfo d = g.si[s];
-    const int32_t L = slice_slots(n);
+// What a block needs of the slice it evaluates.
+struct SliceLane {
+    int64_t p;
+    int32_t ti, n, L, tb, kind;
+};
+__device__ __forceinline__ SliceLane slice_lane(const Geo &g, int64_t s, int lane) {
+    SliceLane v;
+    v.p = 32 * s + lane;
+    v.ti = g.tinfo[v.p];
+    v.n = g.cnt[v.p];
+    v.L = slice_slots(v.n);
     // every particle of a slice belongs to one block (padding: -1)
-    const int32_t tb = __reduce_max_sync(0xffffffffu, ti);
-    const int kind = tb >= 0 ? g.blocks[tb >> 8].kind : PD_MAT_SKIP;
-    pdl_enter();  // before any return: the next kernel may wait for this one only
-    if (kind == PD_MAT_ELASTO_PLASTIC || L > cap || (g.stop && *g.stop)) return;
+    v.tb = __reduce_max_sync(0xffffffffu, v.ti);
+    v.kind = v.tb >= 0 ? g.blocks[v.tb >> 8].kind : PD_MAT_SKIP;
+    return v;
+}
+// Behind the wait: the slice's block takes part (has left the undeformed state).
+__device__ __forceinline__ bool slice_active(const Geo &g, const SliceLane &v) {
+    return v.kind != PD_MAT_SKIP && g.deformed[v.tb >> 8] != 0;
+}
+// A slice that does not, by the warps w, w + step, ...: its flags carry over.
+__device__ __forceinline__ void carry_slice(const SliceLane &v, const SliceInfo &d, int w, int step, int lane,
+                                            const uint32_t *win, uint32_t *wout, double4 *f, int accumulate) {
+    const uint32_t *wi = win + d.word + lane;
+    uint32_t *wo = wout + d.word + lane;
+    for (int32_t c0 = w; 32 * c0 < v.L; c0 += 4 * step) {
+        uint32_t word[4];  // (all loads before the stores, which may alias them for all the compiler knows)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) word[i] = 32 * (c0 + i * step) < v.n ? wi[32 * (c0 + i * step)] : 0u;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (32 * (c0 + i * step) < v.n) wo[32 * (c0 + i * step)] = word[i];
+    }
+    if (w == 0 && !accumulate) f[v.p] = make_double4(0.0, 0.0, 0.0, 0.0);
+}
+
+// The slice's forces, by the whole block.
+template <int NW>
+__device__ __forceinline__ void force_slice(const Geo &g, const double4 *y, const double2 *mth, const uint32_t *win,
+                                            uint32_t *wout, double4 *f, int accumulate, int32_t cap,
+                                            const SliceLane &v, const SliceInfo &d, int w, int lane, double *term) {
+    const int64_t p = v.p;
+    const int32_t ti = v.ti, n = v.n, L = v.L, tb = v.tb;
+    const int kind = v.kind;
     const int32_t words = (L + 31) >> 5;
     uint32_t *brk = reinterpret_cast<uint32_t *>(term + 96 * (int64_t)cap);
     const uint32_t *wi = win + d.word + lane;
     uint32_t *wo = wout + d.word + lane;
-    if (kind == PD_MAT_SKIP || g.deformed[tb >> 8] == 0) {
-        for (int32_t c = w; c < words; c += NW)
-            if (32 * c < n) wo[32 * c] = wi[32 * c];
-        if (w == 0 && !accumulate) f[p] = make_double4(0.0, 0.0, 0.0, 0.0);
-        return;
-    }
     if (accumulate) {
         const double4 f0 = f[lane_record((int32_t)p, ti)];
         const uint64_t nz = 0x8000000000000000ull;
@@ -1017,6 +1038,58 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 1)
     } else if (!accumulate) {
         fo[w] = 0.0;
         if (w == 0) fo[3] = 0.0;
+    }
+}
+
+// SCAN: the S slices from s0 are dealt out to the blocks, whose warps look at
+// a few slices each and carry those over whose body is undeformed; the block
+// then evaluates the others.  (One block per slice, of which an SM holds two, is
+// slow where nothing is to be done: the first steps of a 2.1-million-particle
+// body, undeformed, took 580 us each against 236 with a thread per particle.)
+template <int NW, bool SCAN>
+__global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 1)
+    k_force_slice(Geo g, const double4 *y, const double2 *mth, const uint32_t *win, uint32_t *wout, double4 *f,
+                  int accumulate, int32_t cap, int64_t s0, int64_t S) {
+    extern __shared__ double term[];  // [slot][component][lane], then the broken bits [word][lane]
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if constexpr (!SCAN) {
+        const int64_t s = s0 + blockIdx.x;
+        const SliceLane v = slice_lane(g, s, lane);
+        const SliceInfo d = g.si[s];
+        pdl_enter();  // before any return: the next kernel may wait for this one only
+        if (v.kind == PD_MAT_ELASTO_PLASTIC || v.L > cap || (g.stop && *g.stop)) return;
+        if (slice_active(g, v)) force_slice<NW>(g, y, mth, win, wout, f, accumulate, cap, v, d, w, lane, term);
+        else carry_slice(v, d, w, NW, lane, win, wout, f, accumulate);
+    } else {
+        constexpr int K = 4;  // slices a warp looks at together
+        __shared__ bool todo[NW * K];
+        pdl_enter();
+        if (g.stop && *g.stop) return;
+        const int64_t stride = gridDim.x;
+        for (int64_t i0 = blockIdx.x; i0 < S; i0 += NW * K * stride) {
+            SliceLane v[K];
+            bool mine[K], run[K];
+#pragma unroll
+            for (int j = 0; j < K; ++j) {  // (past the end: the last slice again)
+                v[j] = slice_lane(g, s0 + min(i0 + (w * K + j) * stride, S - 1), lane);
+                mine[j] = i0 + (w * K + j) * stride < S && v[j].kind != PD_MAT_ELASTO_PLASTIC && v[j].L <= cap;
+                run[j] = mine[j] && slice_active(g, v[j]);
+            }
+            for (int j = 0; j < K; ++j) {
+                if (mine[j] && !run[j])
+                    carry_slice(v[j], g.si[v[j].p >> 5], 0, 1, lane, win, wout, f, accumulate);
+                if (lane == 0) todo[w * K + j] = run[j];
+            }
+            __syncthreads();
+            for (int j = 0; j < NW * K; ++j) {
+                if (!todo[j]) continue;  // the same for the whole block
+                const int64_t s = s0 + i0 + j * stride;
+                force_slice<NW>(g, y, mth, win, wout, f, accumulate, cap, slice_lane(g, s, lane), g.si[s], w, lane,
+                                term);
+                __syncthreads();  // the terms are reused
+            }
+            __syncthreads();  // todo is
+        }
     }
 }
 
@@ -1446,26 +1519,29 @@ static void force_slice_attrs() {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || done[dev].load()) return;
     const int bytes = (int)force_slice_bytes(kForceSlots);
-    if (cudaFuncSetAttribute(k_force_slice<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess &&
-        cudaFuncSetAttribute(k_force_slice<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess)
-        done[dev].store(true);
+    bool ok = true;
+    for (auto kern : {k_force_slice<8, false>, k_force_slice<16, false>, k_force_slice<8, true>})
+        ok &= cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+    if (ok) done[dev].store(true);
 }
 
 void launch_force_serial(cudaStream_t st, const Geo &g, const double4 *y, const double2 *mth,
                          const uint32_t *win, uint32_t *wout, double4 *f, int accumulate,
-                         const SerialRun *runs, size_t n_runs) {
+                         const SerialRun *runs, size_t n_runs, bool idle) {
     for (const SerialRun *r = runs; r < runs + n_runs; ++r) {
         const int32_t cap = !r->by_slice ? -1 : r->slots < kForceSlots ? r->slots : kForceSlots;
         const int64_t S = (r->p1 - r->p0) / 32;
         if (r->by_slice) {
             const size_t sm = force_slice_bytes(cap);
             force_slice_attrs();
-            if (wide_slices(S))
-                launch_dep_smem(k_force_slice<16>, (unsigned)S, 512, sm, st, g, y, mth, win, wout, f, accumulate, cap,
-                                r->p0 / 32);
-            else
-                launch_dep_smem(k_force_slice<8>, (unsigned)S, 256, sm, st, g, y, mth, win, wout, f, accumulate, cap,
-                                r->p0 / 32);
+            // (two waves of blocks cost little: 1,024 undeformed slices 11 us)
+            const bool scan = idle && S > 4 * kWideSlices;
+            const bool wide = wide_slices(S);
+            launch_dep_smem(wide   ? k_force_slice<16, false>
+                            : scan ? k_force_slice<8, true>
+                                   : k_force_slice<8, false>,
+                            (unsigned)(scan ? 2 * kWideSlices : S), wide ? 512 : 256, sm, st, g, y, mth, win, wout, f,
+                            accumulate, cap, r->p0 / 32, S);
             pd::note_launch();
         }
         if (r->ep || r->slots > cap) {

@@ -211,9 +211,10 @@ struct SerialRun {
 };
 void launch_theta_serial(cudaStream_t st, const Geo &g, const double4 *y, const uint32_t *win,
                          double2 *mth, const SerialRun *runs, size_t n_runs);
+// idle: some block may be undeformed
 void launch_force_serial(cudaStream_t st, const Geo &g, const double4 *y, const double2 *mth,
                          const uint32_t *win, uint32_t *wout, double4 *f, int accumulate,
-                         const SerialRun *runs, size_t n_runs);
+                         const SerialRun *runs, size_t n_runs, bool idle);
 // elasto_plastic.jl:166-172 out_of_loop! td_norm2 pass (breaks bonds too)
 void launch_td_serial(cudaStream_t st, const Geo &g, const double4 *y, const double2 *mth,
                       const uint32_t *win, uint32_t *wout, int64_t p0, int64_t p1);

@@ -237,10 +237,12 @@ namespace pd {
 //   2,000         21 / 37    38 / 45      50 / 48      59 / 49     198 / 108
 //   8,192         52 / 117   109 / 148    149 / 161    179 / 163   641 / 394
 //  65,536         364 / 1054 807 / 1290   1100 / 1390  1331 / 1395 4741 / 3231
-// The dilatation's blocks do less per slice and its line lies higher (32
-// slots, state-based step with the force by slices: 8,192 slices 228 with
-// threads, 256 without; 65,536: 1844 and 2265).  The elasto-plastic force,
-// whose two visits differ, has the thread form only.
+// The dilatation evaluates a bond once in either form, so that threads win
+// from some 3,500 slices on however long the lists (state-based steps, the
+// force by slices where that is faster, dilatation by threads / slices:
+// 32 slots 2,000 slices 76 / 74, 8,192 228 / 257; 120 slots 2,000 192 / 174,
+// 3,907 309 / 319, 65,536 4768 / 5313).  The elasto-plastic force, whose two
+// visits differ, has the thread form only.
 std::vector<SerialRun> serial_runs(const pd_env *env, size_t b0, size_t b1, bool theta) {
     constexpr size_t kMaxRuns = 8;
     auto takes = [&](const HostBlock &b) {
@@ -255,7 +257,8 @@ std::vector<SerialRun> serial_runs(const pd_env *env, size_t b0, size_t b1, bool
         const HostBlock &b = env->hb[k];
         if (!takes(b) || b.n == 0) continue;
         const bool ep = b.kind == PD_MAT_ELASTO_PLASTIC;
-        const bool by_slice = (theta || !ep) && !(b.mean_slots <= (theta ? 40 : 28) && S >= 300 + 70 * (int64_t)b.mean_slots);
+        const int64_t line = 300 + 70 * (int64_t)b.mean_slots;  // slices from which on threads are faster
+        const bool by_slice = theta ? S < std::min<int64_t>(line, 3500) : !ep && (b.mean_slots > 28 || S < line);
         const int64_t p0 = b.first_int, p1 = p0 + kSlice * slices(b);
         if (by_slice) wide += slices(b);
         if (!runs.empty() && runs.back().p1 == p0 && runs.back().by_slice == by_slice) {
@@ -312,6 +315,8 @@ pd_status update_acc_serial(pd_env *env, bool momentum, const int32_t *stop) {
     if (any_lps)
         launch_theta_serial(st, g, env->y.p, env->words[env->cur].p, env->mth.p, env->theta_runs.data(),
                             env->theta_runs.size());
+    bool idle = false;
+    for (size_t b = 0; b < env->hb.size(); ++b) idle |= env->hb[b].kind != PD_MAT_SKIP && !env->deformed_h[b];
     const SerialRun *runs = env->force_runs.data();
     const size_t n_runs = env->force_runs.size();
     if (any_ep) {
@@ -321,14 +326,14 @@ pd_status update_acc_serial(pd_env *env, bool momentum, const int32_t *stop) {
                          env->N);
         prof_begin(env, st);
         launch_force_serial(st, g, env->y.p, env->mth.p, env->words[1 - env->cur].p, env->words[env->cur].p,
-                            env->f.p, 0, runs, n_runs);
+                            env->f.p, 0, runs, n_runs, idle);
         prof_end(env, st);
         env->ecur = 1 - env->ecur;
     } else {
         // fill!(f, 0) + force_density_T! for every block
         prof_begin(env, st);
         launch_force_serial(st, g, env->y.p, env->mth.p, env->words[env->cur].p, env->words[1 - env->cur].p,
-                            env->f.p, 0, runs, n_runs);
+                            env->f.p, 0, runs, n_runs, idle);
         prof_end(env, st);
         env->cur = 1 - env->cur;
     }
@@ -590,7 +595,7 @@ extern "C" pd_status pd_force_density_device(pd_env *env, int64_t block, double 
     std::vector<int32_t> one(1, 1);
     CK(cudaMemcpyAsync(env->deformed.p + block, one.data(), 4, cudaMemcpyHostToDevice, st));
     launch_force_serial(st, g, env->tmp_y.p, env->mth.p, env->words[env->cur].p, env->words[1 - env->cur].p,
-                        env->tmp_f.p, 1, force.data(), force.size());
+                        env->tmp_f.p, 1, force.data(), force.size(), false);
     int64_t w0 = env->sinfo_h[p0 / 32].word, w1 = env->sinfo_h[p1 / 32].word;
     if (w1 > w0)
         CK(cudaMemcpyAsync(env->words[env->cur].p + w0, env->words[1 - env->cur].p + w0, (w1 - w0) * 4,

@@ -130,3 +130,29 @@ def test_many_alternating_blocks(oracle, larger):
     assert np.array_equal(f, ora.f)
     assert np.array_equal(y, ora.y)
     env.close()
+
+
+@pytest.mark.parametrize("peak", [0.0, 0.03, 40.0])
+@pytest.mark.parametrize("law,factor", [("lps", 2.3), ("pmb", 2.6)])
+def test_bodies_that_are_undeformed_at_first(oracle, law, factor, peak):
+    """Many slices of a body that is undeformed throughout, for the first steps
+    only, or from the start, between two small ones that move; an odd number of
+    evaluations, so both buffers of the bond flags are read."""
+    mats = [block("pmb", (5, 4, 3), 1, 1, -0.02), block(law, (37, 28, 21), 2, 2, 0.0, factor=factor),
+            block("lps", (6, 5, 4), 1, 4, 0.06)]
+    gen = mats[1].general
+    gen.velocity[:] = lattice.gaussian_pulse(gen.x, peak, 4.0e-3) if peak else 0.0
+    env = pb.Env(1, mats, [], [], 2.0e-8)
+    ora = oracle.OracleEnv(mats, [], [], 2.0e-8)
+    for n in (9, 4):
+        pb.velocity_verlet_step(env, nsteps=n)
+        for _ in range(n):
+            ora.vv_step()
+        y, v, f, _ = env.get_state()
+        assert np.array_equal(f, ora.f)
+        assert np.array_equal(v, ora.v)
+        assert np.array_equal(y, ora.y)
+        for b, B in enumerate(ora.blocks):
+            assert np.array_equal(env._family(b)[1], B.intact.astype(bool))
+    assert bool(ora.blocks[1].deformed) == (peak > 0.0)
+    env.close()
