@@ -86,6 +86,7 @@ pd::Geo pd_env::geo() const {
     g.nbr = nbr.p;
     g.fam = fam.p;
     g.deformed = deformed.p;
+    g.sms = sm_count;
     g.stop = nullptr;
     g.td2 = td2.p;
     g.edp_in = edp[ecur].p;
@@ -809,6 +810,7 @@ extern "C" pd_status pd_env_finalize(pd_env *env) {
     cudaStream_t st = env->st;
     SetupClock clk;
 
+    if (env->sm_count == 0) CK(cudaDeviceGetAttribute(&env->sm_count, cudaDevAttrMultiProcessorCount, env->device));
     // --- internal layout ---
     if (env->precision == PD_PREC_FP64) env->unit = bond_unit(env->hb);
     int64_t N = 0;

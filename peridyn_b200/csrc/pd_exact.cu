@@ -833,7 +833,6 @@ __global__ void __launch_bounds__(kThreads)
 // Largest family evaluated in shared memory: 288 slots of 768 bytes and
 // their broken bits, within the 227 KB a block may take.
 constexpr int32_t kForceSlots = 288;
-constexpr int64_t kWideSlices = 148;  // SMs of a B200
 inline size_t force_slice_bytes(int32_t cap) { return 768 * (size_t)cap + 128 * (size_t)((cap + 31) / 32); }
 
 // A particle of a slice the block evaluation does not cover (accumulating).
@@ -1491,14 +1490,14 @@ void launch_weighted_volume(cudaStream_t st, const Geo &g, double2 *mth) {
 // a 990-particle cube 26.9 against 28.3 us per step with eight, a
 // 40,000-particle bar (two blocks of eight on an SM, one of sixteen) 177
 // against 144 us.
-static bool wide_slices(int64_t slices) { return slices <= kWideSlices; }
+static bool wide_slices(const Geo &g, int64_t slices) { return slices <= g.sms; }
 
 void launch_theta_serial(cudaStream_t st, const Geo &g, const double4 *y, const uint32_t *win,
                          double2 *mth, const SerialRun *runs, size_t n_runs) {
     for (const SerialRun *r = runs; r < runs + n_runs; ++r) {
         const int64_t S = (r->p1 - r->p0) / 32;
         if (!r->by_slice) k_theta_serial<<<grid_for(r->p1 - r->p0), kThreads, 0, st>>>(g, y, win, mth, r->p0, r->p1);
-        else if (wide_slices(S)) launch_dep(k_theta_slice<16>, (unsigned)S, 512, st, g, y, win, mth, r->p0 / 32);
+        else if (wide_slices(g, S)) launch_dep(k_theta_slice<16>, (unsigned)S, 512, st, g, y, win, mth, r->p0 / 32);
         else launch_dep(k_theta_slice<8>, (unsigned)S, 256, st, g, y, win, mth, r->p0 / 32);
         pd::note_launch();
     }
@@ -1535,12 +1534,12 @@ void launch_force_serial(cudaStream_t st, const Geo &g, const double4 *y, const 
             const size_t sm = force_slice_bytes(cap);
             force_slice_attrs();
             // (two waves of blocks cost little: 1,024 undeformed slices 11 us)
-            const bool scan = idle && S > 4 * kWideSlices;
-            const bool wide = wide_slices(S);
+            const bool scan = idle && S > 4 * g.sms;
+            const bool wide = wide_slices(g, S);
             launch_dep_smem(wide   ? k_force_slice<16, false>
                             : scan ? k_force_slice<8, true>
                                    : k_force_slice<8, false>,
-                            (unsigned)(scan ? 2 * kWideSlices : S), wide ? 512 : 256, sm, st, g, y, mth, win, wout, f,
+                            (unsigned)(scan ? 2 * g.sms : S), wide ? 512 : 256, sm, st, g, y, mth, win, wout, f,
                             accumulate, cap, r->p0 / 32, S);
             pd::note_launch();
         }

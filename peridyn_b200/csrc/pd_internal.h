@@ -117,6 +117,7 @@ struct Geo {
     const int32_t *nbr;        // bond index data (see SliceInfo)
     const uint32_t *fam;       // family-member bits (same layout as intact)
     const int32_t *deformed;   // per block
+    int32_t sms;               // the device's multiprocessors (launch rules)
     const int32_t *stop;       // not null: the force kernels return at once when *stop is set
     // elasto-plastic blocks: td_norm2 per particle, plastic deviatoric
     // strain per bond slot (read from edp_in, written to edp_out)
