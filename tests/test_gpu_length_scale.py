@@ -74,3 +74,38 @@ def test_lengths_far_from_one(oracle, monkeypatch, layout, law, scale):
 @pytest.mark.parametrize("laws,scale", [(("lps", "ep"), 1e-33), (("pmb", "ep"), 1e38)])
 def test_blocks_of_two_laws(oracle, laws, scale):
     _compare(oracle, [_block(laws[0], scale), _block(laws[1], scale, 2, 40.0)])
+
+
+@pytest.mark.parametrize("scale", [1e-3, 1e-55])
+def test_halo_records_carry_the_displacement_itself(scale):
+    """Packed on one environment, unpacked on another: the same state, in the
+    environment's unit whatever the records' is."""
+    import ctypes
+
+    import torch
+
+    from peridyn_b200 import _abi
+
+    L = _abi.lib()
+    mats = [_block("lps", scale)]
+    src = pb.Env(1, mats, [], [], 1.0, precision="fp64")
+    dst = pb.Env(1, mats, [], [], 1.0, precision="fp64")
+    y, v, f, _ = src.get_state()
+    rng = np.random.default_rng(1)
+    y = np.asfortranarray(y + rng.normal(0.0, 1e-3 * scale, y.shape))
+    v = np.asfortranarray(rng.normal(0.0, scale, y.shape))
+    _abi.check(L.pd_env_set_state(src._h, _abi.dptr(y), _abi.dptr(v), _abi.dptr(f)))
+    pb.update_acc(src)
+    pb.update_acc(dst)
+    n = y.shape[1]
+    idx = torch.arange(n, dtype=torch.int64, device="cuda")
+    buf = torch.zeros(9 * n, dtype=torch.float64, device="cuda")
+    _abi.check(L.pd_env_pack_halo(src._h, ctypes.c_void_p(idx.data_ptr()), n, ctypes.c_void_p(buf.data_ptr())))
+    torch.cuda.synchronize()
+    x = mats[0].general.x
+    assert np.array_equal(buf.cpu().numpy().reshape(n, 9)[:, :3], (y - x).T)
+    _abi.check(L.pd_env_unpack_halo(dst._h, ctypes.c_void_p(idx.data_ptr()), n, ctypes.c_void_p(buf.data_ptr())))
+    for a, b in zip(src.get_state()[:3], dst.get_state()[:3]):
+        assert np.array_equal(a, b)
+    src.close()
+    dst.close()
