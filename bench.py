@@ -592,7 +592,7 @@ def main():
         "hbm_gbs_algorithmic": bytes_step * sim_steps * args.steps / t_total / 1e9,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None, "traffic": traffic,
-                     "kernel": ("k_force_serial" if args.precision == "fp64_serial" else
+                     "kernel": ("k_force_slice" if args.precision == "fp64_serial" else
                                 "k_theta + k_step (dilatation, fused bond force + velocity-Verlet)" if lps else
                                 "k_step (fused bond force + velocity-Verlet), one launch per step"),
                      "bytes_per_launch": bytes_step,
@@ -618,7 +618,8 @@ def main():
     line["config"]["setup_s"] = setup_s
     line["config"]["kernel_shape"] = {"warps_per_slice": shape[0], "unroll": shape[1], "chosen_by":
                                       "PD_KERNEL_SHAPE" if os.environ.get("PD_KERNEL_SHAPE") else "autotuner"}
-    line["config"]["launch_path"] = ("persistent cooperative kernel over flip-free runs" if args.persist else
+    line["config"]["launch_path"] = ("dependent launches, step by step" if args.precision == "fp64_serial" else
+                                     "persistent cooperative kernel over flip-free runs" if args.persist else
                                      "CUDA graphs of 32 steps" if not work["contacts"] else
                                      "CUDA graphs of 32 steps between contact neighbour updates")
     if args.precision == "fp32c" and not lps and not args.no_pipe_peaks:

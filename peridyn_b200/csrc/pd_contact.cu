@@ -347,14 +347,6 @@ __global__ void k_c1_select(int64_t n1, int64_t rows, int64_t first2, const int3
     for (int64_t r = 0; r < rows; ++r) nb[r * n1 + i] = r < n ? (int32_t)(first2 + a[r]) : -1;
 }
 
-// The same in one kernel, a warp per set-1 particle, for rows <= kCand / 2:
-// the lanes test the candidate cells' particles (three neighbouring cells of
-// a grid row are one run of clist), the hits are packed into shared memory,
-// and each hit's rank -- how many hits have a larger index -- is its row.  A
-// full buffer is cut to its rows largest before the walk goes on.  Counts
-// the reverse lists on the way.  (A thread per particle, counting, filling
-// and insertion-sorting, left an impact's thousand particles in reach to a
-// few dozen warps: 242 us against 20 for a 17,000-particle sphere.)
 // Set-1 particles in the box (any order: each is worked on by itself).
 __global__ void k_box_list(int64_t first1, int64_t n1, const double4 *__restrict__ y, Box b,
                            int32_t *__restrict__ list, int32_t *__restrict__ count) {
@@ -362,6 +354,14 @@ __global__ void k_box_list(int64_t first1, int64_t n1, const double4 *__restrict
     if (i < n1 && in_box(b, y[first1 + i])) list[atomicAdd(count, 1)] = (int32_t)i;
 }
 
+// Count, fill and selection in one kernel, a warp per listed set-1 particle,
+// for rows <= kCand / 2: the lanes test the candidate cells' particles (three
+// neighbouring cells of a grid row are one run of clist), the hits are packed
+// into shared memory, and each hit's rank -- how many hits have a larger
+// index -- is its row.  A full buffer is cut to its rows largest before the
+// walk goes on.  Counts the reverse lists on the way.  (A thread per particle, counting, filling
+// and insertion-sorting, left an impact's thousand particles in reach to a
+// few dozen warps: 242 us against 20 for a 17,000-particle sphere.)
 constexpr int kCand = 1024, kSelWarps = 4;
 constexpr int64_t kSelBlocks = 148 * 6;  // 32 KB of buffers a block
 __global__ void __launch_bounds__(32 * kSelWarps)

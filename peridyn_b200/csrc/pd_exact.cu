@@ -823,8 +823,8 @@ __global__ void __launch_bounds__(kThreads)
 //
 // What bounds it: the two blocks an SM holds (94 KB of terms for 122 slots)
 // alternate between evaluation, a chain of some 600 cycles per pair of
-// slots, and the sums, 244 dependent additions of 17 cycles.  FP64 pipe 33 %,
-// issue 47 % busy (48^3 PMB cube).  Against a thread per particle
+// slots, and the sums, 244 dependent additions of 17 cycles.  FP64 pipe 36 %,
+// issue 50 % busy (48^3 PMB cube; state-based 40 and 51 %).  Against a thread per particle
 // that evaluates a bond at each of its two visits: force pass of a
 // 990-particle cube 15 against 198 us, of a 40,000-particle state-based bar
 // 84 against 484 us.  16 warps of 128 registers on an SM; 24 warps of 80

@@ -14,8 +14,8 @@
 // rounding, so y is within one ulp.  a r is within two ulps of a/b, so one
 // correction makes q faithful and the second rounds it.
 //
-// Square root: rsqrt.approx.ftz.f64 is off by at most 2^-18.9 (|1 - a y y|
-// measured: 2^-19.03); one cubic step takes y to a couple of ulps, and the
+// Square root: rsqrt.approx.ftz.f64 is off by at most 2^-18.9 (|1 - a y y|,
+// about twice that, measured: 2^-19.04); one cubic step takes y to a couple of ulps, and the
 // corrected root is sqrt(a) to 2^-100 before its rounding, so it can only be
 // misrounded when sqrt(a) lies that close to the middle of two neighbours.
 // There the (exact) residual a - root^2 is root ulp(root) in magnitude to
