@@ -1181,8 +1181,8 @@ extern "C" pd_status pd_env_finalize(pd_env *env) {
         const int64_t slices = (b.n + kSlice - 1) / kSlice;
         b.mean_slots = slices > 0 ? (int32_t)((walked + slices - 1) / slices) : 0;
     }
-    env->force_runs = serial_runs(env, 0, env->hb.size(), false);
-    env->theta_runs = serial_runs(env, 0, env->hb.size(), true);
+    env->force_runs = serial_runs(env, false);
+    env->theta_runs = serial_runs(env, true);
     // membership bits and list places for the serial mode's fused integration
     if (env->precision == PD_PREC_FP64_SERIAL && !env->hbc.empty() && env->hbc.size() <= (size_t)kMaxFusedBC) {
         std::vector<uint8_t> bits(N, 0);

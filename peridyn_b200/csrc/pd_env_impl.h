@@ -313,8 +313,10 @@ pd_status fast_land_flags(pd_env *env);
 // estimate from particle counts and family rows; for admission control).
 int64_t footprint_estimate(const pd_env *env);
 pd_status fast_update_acc(pd_env *env);
-// Runs of the blocks [b0, b1) for the force or the dilatation.
-std::vector<SerialRun> serial_runs(const pd_env *env, size_t b0, size_t b1, bool theta);
+// How the force or the dilatation of one block, among S slices in all, and
+// of the environment's blocks is evaluated.
+SerialRun serial_run(const HostBlock &b, int64_t S, bool theta);
+std::vector<SerialRun> serial_runs(const pd_env *env, bool theta);
 // momentum: p = m v at the end; stop: see Geo::stop.
 pd_status update_acc_serial(pd_env *env, bool momentum = true, const int32_t *stop = nullptr);
 }  // namespace pd

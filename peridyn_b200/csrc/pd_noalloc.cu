@@ -105,13 +105,13 @@ extern "C" pd_status pd_force_density_device_static(pd_env *env, int64_t block, 
     launch_unpack3(st, hb.n, f_dev + 3 * hb.first_env, map, fs);
     Geo g = env->geo();
     const int64_t p0 = hb.first_int, p1 = hb.first_int + n_pad;
-    const auto theta = serial_runs(env, block, block + 1, true), force = serial_runs(env, block, block + 1, false);
+    const SerialRun theta = serial_run(hb, (p1 - p0) / kSlice, true), force = serial_run(hb, (p1 - p0) / kSlice, false);
     if (hb.kind == PD_MAT_ORDINARY_STATE_BASED)
-        launch_theta_serial(st, g, ys, env->words[env->cur].p, env->mth.p, theta.data(), theta.size());
+        launch_theta_serial(st, g, ys, env->words[env->cur].p, env->mth.p, &theta, 1);
     // force_density_T! has no deformed gate: mark the block active
     CK(cudaMemcpyAsync(env->deformed.p + block, &kOne, sizeof(int32_t), cudaMemcpyHostToDevice, st));
     launch_force_serial(st, g, ys, env->mth.p, env->words[env->cur].p, env->words[1 - env->cur].p, fs, 1,
-                        force.data(), force.size(), false);
+                        &force, 1, false);
     const int64_t w0 = env->sinfo_h[p0 / 32].word, w1 = env->sinfo_h[p1 / 32].word;
     if (w1 > w0)
         CK(cudaMemcpyAsync(env->words[env->cur].p + w0, env->words[1 - env->cur].p + w0, (w1 - w0) * sizeof(uint32_t),

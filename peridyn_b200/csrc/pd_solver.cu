@@ -224,7 +224,7 @@ __global__ void k_clear_idx(int64_t n, const int32_t *__restrict__ idx, int32_t 
 
 namespace pd {
 
-// How the blocks [b0, b1) are evaluated.  A block of warps per slice
+// How a block of an evaluation over S slices in all is evaluated.  A block of warps per slice
 // evaluates every bond once and side by side, but an SM holds two or three of
 // them, each some 4.5 us long however few its slots; a thread per particle
 // evaluates every bond at both visits, one after another.  Short slot lists
@@ -243,30 +243,33 @@ namespace pd {
 // 32 slots 2,000 slices 76 / 74, 8,192 228 / 257; 120 slots 2,000 192 / 174,
 // 3,907 309 / 319, 65,536 4768 / 5313).  The elasto-plastic force, whose two
 // visits differ, has the thread form only.
-std::vector<SerialRun> serial_runs(const pd_env *env, size_t b0, size_t b1, bool theta) {
+SerialRun serial_run(const HostBlock &b, int64_t S, bool theta) {
+    const bool ep = b.kind == PD_MAT_ELASTO_PLASTIC;
+    const int64_t line = 300 + 70 * (int64_t)b.mean_slots;  // slices from which on threads are faster
+    const bool by_slice = theta ? S < std::min<int64_t>(line, 3500) : !ep && (b.mean_slots > 28 || S < line);
+    return SerialRun{b.first_int, b.first_int + (b.n + kSlice - 1) / kSlice * kSlice, b.slots, by_slice, ep};
+}
+
+// Runs of the environment's blocks for the force or the dilatation.
+std::vector<SerialRun> serial_runs(const pd_env *env, bool theta) {
     constexpr size_t kMaxRuns = 8;
     auto takes = [&](const HostBlock &b) {
-        return !theta || b.kind == PD_MAT_ORDINARY_STATE_BASED || b.kind == PD_MAT_ELASTO_PLASTIC;
+        return b.n > 0 && (!theta || b.kind == PD_MAT_ORDINARY_STATE_BASED || b.kind == PD_MAT_ELASTO_PLASTIC);
     };
-    auto slices = [](const HostBlock &b) { return (b.n + kSlice - 1) / kSlice; };
     int64_t S = 0, wide = 0;
-    for (size_t k = b0; k < b1; ++k)
-        if (takes(env->hb[k])) S += slices(env->hb[k]);
+    for (const auto &b : env->hb)
+        if (takes(b)) S += (b.n + kSlice - 1) / kSlice;
     std::vector<SerialRun> runs;
-    for (size_t k = b0; k < b1; ++k) {
-        const HostBlock &b = env->hb[k];
-        if (!takes(b) || b.n == 0) continue;
-        const bool ep = b.kind == PD_MAT_ELASTO_PLASTIC;
-        const int64_t line = 300 + 70 * (int64_t)b.mean_slots;  // slices from which on threads are faster
-        const bool by_slice = theta ? S < std::min<int64_t>(line, 3500) : !ep && (b.mean_slots > 28 || S < line);
-        const int64_t p0 = b.first_int, p1 = p0 + kSlice * slices(b);
-        if (by_slice) wide += slices(b);
-        if (!runs.empty() && runs.back().p1 == p0 && runs.back().by_slice == by_slice) {
-            runs.back().p1 = p1;
-            runs.back().slots = std::max(runs.back().slots, b.slots);
-            runs.back().ep |= ep;
+    for (const auto &b : env->hb) {
+        if (!takes(b)) continue;
+        const SerialRun r = serial_run(b, S, theta);
+        if (r.by_slice) wide += (r.p1 - r.p0) / kSlice;
+        if (!runs.empty() && runs.back().p1 == r.p0 && runs.back().by_slice == r.by_slice) {
+            runs.back().p1 = r.p1;
+            runs.back().slots = std::max(runs.back().slots, r.slots);
+            runs.back().ep |= r.ep;
         } else {
-            runs.push_back(SerialRun{p0, p1, b.slots, by_slice, ep});
+            runs.push_back(r);
         }
     }
     if (runs.size() <= kMaxRuns) return runs;
@@ -588,14 +591,14 @@ extern "C" pd_status pd_force_density_device(pd_env *env, int64_t block, double 
     launch_unpack3(st, hb.n, f_dev + 3 * hb.first_env, map, env->tmp_f.p);
     Geo g = env->geo();
     int64_t p0 = hb.first_int, p1 = hb.first_int + ((hb.n + 31) / 32) * 32;
-    const auto theta = serial_runs(env, block, block + 1, true), force = serial_runs(env, block, block + 1, false);
+    const SerialRun theta = serial_run(hb, (p1 - p0) / kSlice, true), force = serial_run(hb, (p1 - p0) / kSlice, false);
     if (hb.kind == PD_MAT_ORDINARY_STATE_BASED)
-        launch_theta_serial(st, g, env->tmp_y.p, env->words[env->cur].p, env->mth.p, theta.data(), theta.size());
+        launch_theta_serial(st, g, env->tmp_y.p, env->words[env->cur].p, env->mth.p, &theta, 1);
     // force_density_T! itself has no gate: compute unconditionally
     std::vector<int32_t> one(1, 1);
     CK(cudaMemcpyAsync(env->deformed.p + block, one.data(), 4, cudaMemcpyHostToDevice, st));
     launch_force_serial(st, g, env->tmp_y.p, env->mth.p, env->words[env->cur].p, env->words[1 - env->cur].p,
-                        env->tmp_f.p, 1, force.data(), force.size(), false);
+                        env->tmp_f.p, 1, &force, 1, false);
     int64_t w0 = env->sinfo_h[p0 / 32].word, w1 = env->sinfo_h[p1 / 32].word;
     if (w1 > w0)
         CK(cudaMemcpyAsync(env->words[env->cur].p + w0, env->words[1 - env->cur].p + w0, (w1 - w0) * 4,

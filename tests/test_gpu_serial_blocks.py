@@ -30,10 +30,10 @@ def block(law, dims, ntypes, first_type, offset, factor=2.3, seed=5):
     return pb.PeridynamicsMaterial(gen, pb.OrdinaryStateBasedSpecific(list(20e9 * r), list(9e9 * r), cs, rho))
 
 
-def three_blocks(law, sizes):
+def three_blocks(law, sizes, factor=2.3):
     other = "lps" if law == "pmb" else "pmb"
-    return [block(other, sizes[0], 3, 1, 0.0), block(law, sizes[1], 2, 4, 0.03, seed=6),
-            block(law, sizes[2], 5, 6, 0.06, seed=7)]
+    return [block(other, sizes[0], 3, 1, 0.0, factor), block(law, sizes[1], 2, 4, 0.03, factor, seed=6),
+            block(law, sizes[2], 5, 6, 0.06, factor, seed=7)]
 
 
 @pytest.mark.parametrize("law", ["pmb", "lps"])
@@ -59,7 +59,8 @@ def test_blocks_of_several_types(oracle, law, sizes):
 
 @pytest.mark.parametrize("entry", ["pd_force_density_device_static", "pd_force_density_device"])
 @pytest.mark.parametrize("law", ["pmb", "lps"])
-def test_one_block_of_several_through_device_pointers(oracle, law, entry):
+@pytest.mark.parametrize("dims,factor", [((9, 7, 5), 2.3), ((36, 32, 32), 1.1)])  # a block per slice, a thread each
+def test_one_block_of_several_through_device_pointers(oracle, law, dims, factor, entry):
     """Each block by itself, in turn; the other blocks' positions are NaN."""
     import ctypes
 
@@ -67,7 +68,7 @@ def test_one_block_of_several_through_device_pointers(oracle, law, entry):
 
     from peridyn_b200 import _abi
 
-    mats = three_blocks(law, ((7, 3, 3), (9, 7, 5), (3, 3, 3)))
+    mats = three_blocks(law, ((7, 3, 3), dims, (3, 3, 3)), factor)
     env = pb.Env(1, mats, [], [], 2.0e-8)
     ora = oracle.OracleEnv(mats, [], [], 2.0e-8)
     rng = np.random.default_rng(4)
