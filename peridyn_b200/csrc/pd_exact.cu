@@ -1533,8 +1533,10 @@ void launch_force_serial(cudaStream_t st, const Geo &g, const double4 *y, const 
         if (r->by_slice) {
             const size_t sm = force_slice_bytes(cap);
             force_slice_attrs();
-            // (two waves of blocks cost little: 1,024 undeformed slices 11 us)
-            const bool scan = idle && S > 4 * g.sms;
+            // (a few waves of blocks cost little -- 2,000 undeformed slices 46
+            // against 44 us per step -- and the scanning kernel is the slower
+            // one for a body that moves: 1,250 slices 95 against 85 us)
+            const bool scan = idle && S > 16 * g.sms;
             const bool wide = wide_slices(g, S);
             launch_dep_smem(wide   ? k_force_slice<16, false>
                             : scan ? k_force_slice<8, true>

@@ -133,13 +133,13 @@ def test_many_alternating_blocks(oracle, larger):
     env.close()
 
 
-@pytest.mark.parametrize("peak", [0.0, 0.03, 40.0])
+@pytest.mark.parametrize("peak", [0.0, 0.1, 40.0])
 @pytest.mark.parametrize("law,factor", [("lps", 2.3), ("pmb", 2.6)])
 def test_bodies_that_are_undeformed_at_first(oracle, law, factor, peak):
     """Many slices of a body that is undeformed throughout, for the first steps
     only, or from the start, between two small ones that move; an odd number of
     evaluations, so both buffers of the bond flags are read."""
-    mats = [block("pmb", (5, 4, 3), 1, 1, -0.02), block(law, (37, 28, 21), 2, 2, 0.0, factor=factor),
+    mats = [block("pmb", (5, 4, 3), 1, 1, -0.02), block(law, (48, 44, 37), 2, 2, 0.0, factor=factor),
             block("lps", (6, 5, 4), 1, 4, 0.06)]
     gen = mats[1].general
     gen.velocity[:] = lattice.gaussian_pulse(gen.x, peak, 4.0e-3) if peak else 0.0
